@@ -814,56 +814,6 @@ struct PairLoadTile {
     __device__ __forceinline__ void put_pi(const H3<float> &h) const { st_h(g.pi, pos, n, h); }
 };
 
-// Edge tiles: halo cells outside the lattice take the clamped neighbour,
-// each coordinate clamped on its own (corners included). Sources are cells of
-// the lattice, which no thread writes here, so one pass suffices. A box of
-// ROWS rows holds the tile's rows 1 .. ROWS-2 between two halo rows; the
-// halo columns are LO (column -1 of the tile) and LO + 33 (column 32). UT is
-// the link element, PT the phi element; 9 components of each.
-template <class UT, class PT, int ROWS, int UC, int ULO, int PC, int PLO>
-__device__ __forceinline__ void fill_edge_halo(UT *ux, UT *uy, PT *ph, bool top, bool bottom,
-                                               bool left, bool right) {
-    constexpr int ROW = 34, COL = ROWS;  // cells per halo row / halo column
-    constexpr int CELLS = 2 * ROW + 2 * COL;
-    for (int w = threadIdx.x; w < 9 * 2 * CELLS; w += blockDim.x) {
-        const int k = w / (2 * CELLS);
-        int cell = w - k * (2 * CELLS);
-        const bool link = cell < CELLS;
-        if (!link) cell -= CELLS;
-        const int cols = link ? UC : PC;
-        const int c_lo = link ? ULO : PLO, c_hi = c_lo + 33;
-        int j, m;
-        bool edge;
-        if (cell < 2 * ROW) {
-            const int side = cell / ROW;
-            j = side ? ROWS - 1 : 0;
-            m = c_lo + cell % ROW;
-            edge = side ? bottom : top;
-        } else {
-            cell -= 2 * ROW;
-            const int side = cell / COL;
-            j = cell % COL;
-            m = side ? c_hi : c_lo;
-            edge = side ? right : left;
-        }
-        if (!edge) continue;
-        int sj = j, sm = m;
-        if (top && j == 0) sj = 1;
-        if (bottom && j == ROWS - 1) sj = ROWS - 2;
-        if (left && m == c_lo) sm = c_lo + 1;
-        if (right && m == c_hi) sm = c_hi - 1;
-        if (link) {
-            constexpr int KU = ROWS * UC;
-            const int d = k * KU + j * cols + m, s = k * KU + sj * cols + sm;
-            ux[d] = ux[s];
-            uy[d] = uy[s];
-        } else {
-            constexpr int KP = ROWS * PC;
-            ph[k * KP + j * cols + m] = ph[k * KP + sj * cols + sm];
-        }
-    }
-}
-
 // Edge tiles, one warp: the halo cells of the box rows r .. r+2 that warp r
 // reads (its tile row and the rows on either side) take the clamped
 // neighbour, each coordinate clamped on its own. Sources are lattice cells,
@@ -1101,19 +1051,23 @@ __global__ void __launch_bounds__(256, 1)
 }
 
 // ---------------------------------------------------------------------------
-// FP64 step with the fields staged in shared memory by TMA: one block of 128
-// threads per tile of 4 rows (x) x 32 columns (y), one thread per site, two
-// blocks resident per SM (one stage each, so one block's loads overlap the
-// other's arithmetic). The stage holds
-//   Ux, Uy   [9][6][34] complex   rows ix0-1 .. ix0+4, columns iy0-1 .. iy0+32
-//   phi      [9][6][36] real      rows ix0-1 .. ix0+4, columns iy0-2 .. iy0+33
-//   E1, E2   [8][4][32], pi [9][4][32]   the tile's own sites
-// with edge halos clamped as in the FP32 tile kernel. The per-site code is
-// the one of the global-memory kernel (leapfrog_full_core); results go to
-// global memory from registers (E and pi in place).
+// FP64 step with the fields staged in shared memory by TMA: one block per
+// tile of 2 rows (x) x 32 columns (y), two threads per site (the x and the y
+// direction: lanes l and l + 16 of a warp share site l). A thread then fits
+// in 128 registers without spilling, and three 128-thread blocks (12 warps)
+// share an SM, some loading while others compute. The stage holds
+//   Ux, Uy   [9][4][34] complex  rows ix0-1 .. ix0+2, columns iy0-1 .. iy0+32
+//   phi      [9][4][36] real     rows ix0-1 .. ix0+2, columns iy0-2 .. iy0+33
+//   E1, E2   [8][2][32], pi [9][2][32]   the tile's own sites
+// Results go to global memory from registers (E and pi in place).
+// Bound by the FP64 pipe (about 60% busy at 512^2) and the wait for the
+// stage. us a step at 64^2, 128^2, 256^2, 512^2, 1024^2: one thread a site on
+// 4 x 32 tiles 11.5, 12.3, 24.6, 77.0, 258.8; this kernel 6.2, 9.1, 18.8,
+// 65.3, 232.2. Tiles of 4 rows (two blocks an SM): 8.2, 9.0, 20.6, 67.2,
+// 230.1; of 1 row: 6.2, 10.2, 20.4, 67.8, 244.2.
 // ---------------------------------------------------------------------------
 namespace tile64 {
-constexpr int R = 4, Cn = 32;
+constexpr int R = 2, Cn = 32;
 constexpr int UR = R + 2, UC = Cn + 2;  // link box
 constexpr int PR = R + 2, PC = Cn + 4;  // phi box
 constexpr int kU = UR * UC, kP = PR * PC, kS = R * Cn;
@@ -1126,15 +1080,12 @@ constexpr int PI = E2 + tile::round128(8 * kS * 8);
 constexpr int STAGE = PI + tile::round128(9 * kS * 8);
 constexpr uint32_t TX_BYTES = 2 * 9 * kU * 16 + 9 * kP * 8 + 2 * 8 * kS * 8 + 9 * kS * 8;
 constexpr int SMEM = STAGE + 64 + 128;
-static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two blocks per SM");
+constexpr int THREADS = 2 * R * Cn;
+static_assert(3 * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
 }  // namespace tile64
 
-// Loads from the stage (shared memory) by 32-bit address; the thread sits at
-// row r, column c. bl and bp point at the (-1, -1) corner of its 3 x 3
-// neighbourhood in the link and phi boxes, bs at its own cell of the
-// site-local boxes. The loads are explicit shared-memory instructions, so a
-// link loaded twice is read twice rather than kept live in registers; E and
-// pi are written to global memory in place.
+// Explicit shared-memory loads by 32-bit address, so that a link used twice
+// is read twice rather than kept live in registers.
 __device__ __forceinline__ C<double> lds_c64(uint32_t a) {
     double re, im;
     asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(re), "=d"(im) : "r"(a));
@@ -1145,64 +1096,146 @@ __device__ __forceinline__ double lds_f64(uint32_t a) {
     asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
     return v;
 }
-
-struct FullLoadTile64 {
-    uint32_t bl, bp, bs;
-    const State<double> &g;
-    size_t pos, n;
-    __device__ __forceinline__ FullLoadTile64(uint32_t stage, int r, int c,
-                                              const State<double> &g_, size_t pos_, size_t n_)
-        : bl(stage + (uint32_t)((r * tile64::UC + c) * 16)),
-          bp(stage + tile64::PHI + (uint32_t)((r * tile64::PC + c + 1) * 8)),
-          bs(stage + (uint32_t)((r * tile64::Cn + c) * 8)),
-          g(g_), pos(pos_), n(n_) {}
-    template <int F, int DX, int DY>
-    __device__ __forceinline__ M3<double> link() const {
-        constexpr uint32_t o =
-            (F == kLy ? tile64::UY : tile64::UX) + ((DX + 1) * tile64::UC + DY + 1) * 16;
-        M3<double> m;
+template <int PLANE>  // a matrix whose entries are PLANE bytes apart
+__device__ __forceinline__ M3<double> lds_m3(uint32_t a) {
+    M3<double> m;
 #pragma unroll
-        for (int k = 0; k < 9; k++) m.m[k] = lds_c64(bl + o + k * tile64::kU * 16);
-        return m;
-    }
-    static __device__ __forceinline__ H3<double> h9(uint32_t a, uint32_t S) {
-        H3<double> h;
-        h.d0 = lds_f64(a);
-        h.d1 = lds_f64(a + S);
-        h.d2 = lds_f64(a + 2 * S);
-        h.o01 = {lds_f64(a + 3 * S), lds_f64(a + 4 * S)};
-        h.o02 = {lds_f64(a + 5 * S), lds_f64(a + 6 * S)};
-        h.o12 = {lds_f64(a + 7 * S), lds_f64(a + 8 * S)};
-        return h;
-    }
-    static __device__ __forceinline__ H3<double> h8(uint32_t a) {
-        constexpr uint32_t S = tile64::kS * 8;
-        H3<double> h;
-        h.d0 = lds_f64(a);
-        h.d1 = lds_f64(a + S);
-        h.d2 = -(h.d0 + h.d1);
-        h.o01 = {lds_f64(a + 2 * S), lds_f64(a + 3 * S)};
-        h.o02 = {lds_f64(a + 4 * S), lds_f64(a + 5 * S)};
-        h.o12 = {lds_f64(a + 6 * S), lds_f64(a + 7 * S)};
-        return h;
-    }
-    template <int DX, int DY>
-    __device__ __forceinline__ H3<double> phi() const {
-        return h9(bp + ((DX + 1) * tile64::PC + DY + 1) * 8, tile64::kP * 8);
-    }
-    __device__ __forceinline__ H3<double> pi() const { return h9(bs + tile64::PI, tile64::kS * 8); }
-    __device__ __forceinline__ H3<double> e1() const { return h8(bs + tile64::E1); }
-    __device__ __forceinline__ H3<double> e2() const { return h8(bs + tile64::E2); }
-    __device__ __forceinline__ void put_e(const H3<double> &a, const H3<double> &b) const {
-        st_h8(g.e1, pos, n, a);
-        st_h8(g.e2, pos, n, b);
-    }
-    __device__ __forceinline__ void put_pi(const H3<double> &h) const { st_h(g.pi, pos, n, h); }
-};
+    for (int k = 0; k < 9; k++) m.m[k] = lds_c64(a + k * PLANE);
+    return m;
+}
+template <int PLANE>
+__device__ __forceinline__ H3<double> lds_h(uint32_t a) {
+    H3<double> h;
+    h.d0 = lds_f64(a);
+    h.d1 = lds_f64(a + PLANE);
+    h.d2 = lds_f64(a + 2 * PLANE);
+    h.o01 = {lds_f64(a + 3 * PLANE), lds_f64(a + 4 * PLANE)};
+    h.o02 = {lds_f64(a + 5 * PLANE), lds_f64(a + 6 * PLANE)};
+    h.o12 = {lds_f64(a + 7 * PLANE), lds_f64(a + 8 * PLANE)};
+    return h;
+}
+template <int PLANE>
+__device__ __forceinline__ H3<double> lds_h8(uint32_t a) {
+    H3<double> h;
+    h.d0 = lds_f64(a);
+    h.d1 = lds_f64(a + PLANE);
+    h.d2 = -(h.d0 + h.d1);
+    h.o01 = {lds_f64(a + 2 * PLANE), lds_f64(a + 3 * PLANE)};
+    h.o02 = {lds_f64(a + 4 * PLANE), lds_f64(a + 5 * PLANE)};
+    h.o12 = {lds_f64(a + 6 * PLANE), lds_f64(a + 7 * PLANE)};
+    return h;
+}
 
-// One 4 x 32 tile of the FP64 step: load the stage, wait, clamp the halo on
+__device__ __forceinline__ double other_role(double v) {
+    return __shfl_xor_sync(0xffffffffu, v, 16);
+}
+__device__ __forceinline__ H3<double> other_role(const H3<double> &h) {
+    return {other_role(h.d0),
+            other_role(h.d1),
+            other_role(h.d2),
+            {other_role(h.o01.r), other_role(h.o01.i)},
+            {other_role(h.o02.r), other_role(h.o02.i)},
+            {other_role(h.o12.r), other_role(h.o12.i)}};
+}
+
+// One direction d of one site (dir 0: d = x, o = y; 1: d = y, o = x) from the
+// stage: r, c are the site's row and column in the tile. Both directions run
+// this code on their own addresses. They exchange U_d U_o(+d) for the
+// plaquette and the transported phi for pi, which the x thread updates. Every
+// product is formed as in leapfrog_full_core (same operands, same order), so
+// the bits are the plain-load kernel's.
+__device__ __forceinline__ void leapfrog_role64(uint32_t st, int r, int c, int dir,
+                                                const StepCoef<double> &cf,
+                                                const State<double> &g, C<double> *u_out,
+                                                double *phi_out, int N, int ix, int iy) {
+    constexpr int KU = tile64::kU * 16, KP = tile64::kP * 8, KS = tile64::kS * 8;
+    const size_t n = (size_t)N * N, pos = (size_t)ix * N + iy;
+    const uint32_t cell = (uint32_t)(((r + 1) * tile64::UC + c + 1) * 16);
+    const uint32_t ud = st + (dir ? tile64::UY : tile64::UX) + cell;
+    const uint32_t uo = st + (dir ? tile64::UX : tile64::UY) + cell;
+    // byte offsets to the neighbours at +d, -d and -o, zero where the lattice
+    // ends (clamped neighbours, Lattice.cpp:19-28): cells outside the lattice,
+    // which the TMA filled with zeros, are never read
+    const int id = dir ? iy : ix, io = dir ? ix : iy;
+    const int su = dir ? 16 : 16 * tile64::UC, sp = dir ? 8 : 8 * tile64::PC;
+    const int pd = id + 1 < N ? su : 0, md = id > 0 ? -su : 0;
+    const int mo = io > 0 ? (dir ? -16 * tile64::UC : -16) : 0;
+    const uint32_t ph = st + tile64::PHI + (uint32_t)(((r + 1) * tile64::PC + c + 2) * 8);
+    const int ppd = id + 1 < N ? sp : 0, pmd = id > 0 ? -sp : 0;
+    const uint32_t own = st + (uint32_t)((r * tile64::Cn + c) * 8);
+    double *const e_out = dir ? g.e2 : g.e1;
+
+    if (cf.do_pe) {
+        H3<double> t;
+        {
+            // U12 = (Ux Uy(+x)) (Uy Ux(+y))^dag; the x thread holds the first
+            // factor, the y thread the second
+            const M3<double> mine = mul(lds_m3<KU>(ud), lds_m3<KU>(uo + pd));
+            M3<double> a, b;
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                const C<double> theirs = {other_role(mine.m[k].r), other_role(mine.m[k].i)};
+                a.m[k] = dir ? theirs : mine.m[k];
+                b.m[k] = dir ? mine.m[k] : theirs;
+            }
+            t = i_antiherm(mul_nd(a, b));
+        }
+        {
+            // U_d U_o(+d-o)^dag U_d(-o)^dag U_o(-o), plus (x) or minus (y) U12
+            const M3<double> p = mul_nd(lds_m3<KU>(ud), lds_m3<KU>(uo + pd + mo));
+            const M3<double> q = mul_dn(lds_m3<KU>(ud + mo), lds_m3<KU>(uo + mo));
+            H3<double> s = i_antiherm_mul(p, q);
+            h_axpy(s, dir ? -1. : 1., t);
+            t = s;
+        }
+        h_traceless(t);
+        H3<double> e = lds_h8<KS>(own + (dir ? tile64::E2 : tile64::E1));
+        h_axpy(e, cf.c_e, t);
+        H3<double> br;
+        {
+            const H3<double> pt = conj_h(lds_m3<KU>(ud), lds_h<KP>(ph + ppd));
+            h_axpy(e, cf.c_pi, i_commutator(pt, lds_h<KP>(ph)));
+            br = pt;
+            h_add(br, other_role(pt));
+        }
+        h_traceless(e);
+        st_h8(e_out, pos, n, e);
+        {
+            const H3<double> pt = conj_h_dag(lds_m3<KU>(ud + md), lds_h<KP>(ph + pmd));
+            const H3<double> theirs = other_role(pt);
+            if (dir == 0) {
+                H3<double> pi = lds_h<KS>(own + tile64::PI);
+                const H3<double> phi = lds_h<KP>(ph);
+                h_add(br, pt);
+                h_add(br, theirs);
+                h_axpy(br, -4., phi);
+                h_axpy(pi, cf.c_pi, br);
+                st_h(g.pi, pos, n, pi);
+                if (cf.do_pu) {
+                    H3<double> phin = phi;
+                    h_axpy(phin, cf.c_phi, pi);
+                    st_h(phi_out, pos, n, phin);
+                }
+            }
+        }
+        if (cf.do_pu) {
+            st_m3(u_out, pos, n, taylor2_update(e, cf.c_u, lds_m3<KU>(ud)));
+        }
+    } else if (cf.do_pu) {
+        // phi and U only (the tau = 0 half step, Evolution.cpp:393-394)
+        if (dir == 0) {
+            H3<double> phin = lds_h<KP>(ph);
+            h_axpy(phin, cf.c_phi, lds_h<KS>(own + tile64::PI));
+            st_h(phi_out, pos, n, phin);
+        }
+        st_m3(u_out, pos, n,
+              taylor2_update(lds_h8<KS>(own + (dir ? tile64::E2 : tile64::E1)), cf.c_u, lds_m3<KU>(ud)));
+    }
+}
+
+// One 2 x 32 tile of the FP64 step: load the stage, wait, clamp the halo on
 // edge tiles, advance the tile's sites. tx, ty: the tile in the event's
-// N/4 x N/32 grid.
+// N/2 x N/32 grid.
 template <bool GLOBAL_MAPS>
 __device__ __forceinline__ void tile64_body(const LoadMaps *maps, int N, int tx, int ty,
                                             const StepCoef<double> &cf, double *status,
@@ -1213,9 +1246,8 @@ __device__ __forceinline__ void tile64_body(const LoadMaps *maps, int N, int tx,
     unsigned char *smem = smem_raw + pad;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + tile64::STAGE);
     int *abort_flag = reinterpret_cast<int *>(full + 1);
-    const int tiles_y = N / tile64::Cn, tiles_x = N / tile64::R;
     const int iy0 = ty * tile64::Cn, ix0 = tx * tile64::R;
-    const int tid = threadIdx.x, r = tid >> 5, c = tid & 31;
+    const int tid = threadIdx.x;
     if (tid == 0) {
         mbar_init(full, 1);
         *abort_flag = 0;
@@ -1244,32 +1276,15 @@ __device__ __forceinline__ void tile64_body(const LoadMaps *maps, int N, int tx,
         if (tid == 0 && status) *status = 1.0;
         return;
     }
-    const bool top = tx == 0, bottom = tx == tiles_x - 1;
-    const bool left = ty == 0, right = ty == tiles_y - 1;
-    if (top || bottom || left || right) {
-        fill_edge_halo<C<double>, double, tile64::UR, tile64::UC, 0, tile64::PC, 1>(
-            reinterpret_cast<C<double> *>(smem + tile64::UX),
-            reinterpret_cast<C<double> *>(smem + tile64::UY),
-            reinterpret_cast<double *>(smem + tile64::PHI), top, bottom, left, right);
-        __syncthreads();
-    }
-    const size_t n = (size_t)N * N;
-    const size_t pos = (size_t)(ix0 + r) * N + iy0 + c;
-    const FullLoadTile64 ld(smem_addr(smem), r, c, s, pos, n);
-    M3<double> nx, ny;
-    H3<double> phin;
-    leapfrog_full_core<double, false>(ld, cf, nx, ny, phin);
-    if (cf.do_pu) {
-        st_h(phi_out, pos, n, phin);
-        st_m3(ux_out, pos, n, nx);
-        st_m3(uy_out, pos, n, ny);
-    }
+    // a warp is 16 sites of one row: lanes 0-15 direction x, 16-31 direction y
+    const int w = tid >> 5, dir = (tid >> 4) & 1;
+    const int r = w >> 1, c = (w & 1) * 16 + (tid & 15);
+    leapfrog_role64(smem_addr(smem), r, c, dir, cf, s, dir ? uy_out : ux_out, phi_out, N,
+                        ix0 + r, iy0 + c);
 }
 
-// (128, 1): ptxas then fits the site in 190 registers without spilling (with
-// a stated minimum of 2 blocks it used 255 and spilled), and two blocks per SM
-// still fit in registers and shared memory
-__global__ void __launch_bounds__(128, 1)
+// (THREADS, 3): what shared memory allows, 168 registers a thread
+__global__ void __launch_bounds__(tile64::THREADS, 3)
     k_leapfrog_tile64(const __grid_constant__ LoadMaps maps, int N, StepCoef<double> cf,
                       double *status, State<double> s, C<double> *ux_out, C<double> *uy_out,
                       double *phi_out) {
@@ -1278,10 +1293,10 @@ __global__ void __launch_bounds__(128, 1)
                        ux_out, uy_out, phi_out);
 }
 
-// The FP64 batch over the TMA tiles: one block per 4 x 32 tile of the
-// concatenated tile lists; the block reads its event's descriptor and tensor
-// maps from global memory.
-__global__ void __launch_bounds__(128, 1)
+// The FP64 batch over the TMA tiles: one block per tile of the concatenated
+// tile lists; the block reads its event's descriptor and tensor maps from
+// global memory.
+__global__ void __launch_bounds__(tile64::THREADS, 3)
     k_leapfrog_tile64_batch(const BatchEvent<double> *__restrict__ evs, int n_events,
                             const int *__restrict__ tile_begin, const LoadMaps *__restrict__ maps,
                             double *status) {
@@ -1391,7 +1406,8 @@ int batch_max_blocks_per_sm(int variant, int n_events) {
         } else {
             cudaFuncSetAttribute(k_leapfrog_tile64_batch,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, tile64::SMEM);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile64_batch, 128,
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile64_batch,
+                                                          tile64::THREADS,
                                                           tile64::SMEM);
             return nb > 0 ? 1 : 0;  // one block per tile: the grid is the tile count
         }
@@ -1413,7 +1429,7 @@ void launch_leapfrog_batch(const BatchEvent<T> *d_evs, int n_events, const int *
             k_leapfrog_tile_batch<<<grid < total_tiles ? grid : total_tiles, 256, smem, st>>>(
                 d_evs, n_events, d_tile_begin, total_tiles, d_maps, status, 4u);
         } else {
-            k_leapfrog_tile64_batch<<<total_tiles, 128, tile64::SMEM, st>>>(
+            k_leapfrog_tile64_batch<<<total_tiles, tile64::THREADS, tile64::SMEM, st>>>(
                 d_evs, n_events, d_tile_begin, d_maps, status);
         }
         return;
@@ -1484,18 +1500,26 @@ bool encode_step_maps<float>(int N, const State<float> &s, LoadMaps *m) {
            encode_tiled_3d(&m->pi, s.pi, U32, 4, n, n, 9, Cn, R, 9);
 }
 
-template <>
-bool encode_step_maps<double>(int N, const State<double> &s, LoadMaps *m) {
-    using namespace tile64;
+namespace {
+
+// links and phi from `a`, E and pi from `b`; a complex link entry is two
+// 8-byte words
+bool encode_maps64(int N, const State<double> &a, const State<double> &b, LoadMaps *m) {
     const uint64_t n = (uint64_t)N;
     const auto U64 = CU_TENSOR_MAP_DATA_TYPE_UINT64;
-    // a complex link entry is two 8-byte words
-    return encode_tiled_3d(&m->ux, s.ux, U64, 8, 2 * n, n, 9, 2 * UC, UR, 9) &&
-           encode_tiled_3d(&m->uy, s.uy, U64, 8, 2 * n, n, 9, 2 * UC, UR, 9) &&
-           encode_tiled_3d(&m->phi, s.phi, U64, 8, n, n, 9, PC, PR, 9) &&
-           encode_tiled_3d(&m->e1, s.e1, U64, 8, n, n, 8, Cn, R, 8) &&
-           encode_tiled_3d(&m->e2, s.e2, U64, 8, n, n, 8, Cn, R, 8) &&
-           encode_tiled_3d(&m->pi, s.pi, U64, 8, n, n, 9, Cn, R, 9);
+    return encode_tiled_3d(&m->ux, a.ux, U64, 8, 2 * n, n, 9, 2 * tile64::UC, tile64::UR, 9) &&
+           encode_tiled_3d(&m->uy, a.uy, U64, 8, 2 * n, n, 9, 2 * tile64::UC, tile64::UR, 9) &&
+           encode_tiled_3d(&m->phi, a.phi, U64, 8, n, n, 9, tile64::PC, tile64::PR, 9) &&
+           encode_tiled_3d(&m->e1, b.e1, U64, 8, n, n, 8, tile64::Cn, tile64::R, 8) &&
+           encode_tiled_3d(&m->e2, b.e2, U64, 8, n, n, 8, tile64::Cn, tile64::R, 8) &&
+           encode_tiled_3d(&m->pi, b.pi, U64, 8, n, n, 9, tile64::Cn, tile64::R, 9);
+}
+
+}  // namespace
+
+template <>
+bool encode_step_maps<double>(int N, const State<double> &s, LoadMaps *m) {
+    return encode_maps64(N, s, s, m);
 }
 
 namespace {
@@ -1539,15 +1563,19 @@ bool use_tile64_kernel() {
     return tile;
 }
 
-bool launch_leapfrog_tile64(int N, const State<double> &s, C<double> *ux_out, C<double> *uy_out,
+// One FP64 step on the tiles: links and phi from `links`, E and pi from `ein`,
+// E and pi written to `out`, the new links and phi to the pointers. False if a
+// tensor map could not be encoded (nothing launched).
+bool launch_leapfrog_tile64(int N, const State<double> &links, const State<double> &ein,
+                            const State<double> &out, C<double> *ux_out, C<double> *uy_out,
                             double *phi_out, const StepCoef<double> &cf, double *status,
                             cudaStream_t st) {
     using namespace tile64;
     LoadMaps m;
-    if (!encode_step_maps<double>(N, s, &m)) return false;
+    if (!encode_maps64(N, links, ein, &m)) return false;
     cudaFuncSetAttribute(k_leapfrog_tile64, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    k_leapfrog_tile64<<<(N / R) * (N / Cn), 128, SMEM, st>>>(m, N, cf, status, s, ux_out, uy_out,
-                                                               phi_out);
+    k_leapfrog_tile64<<<(N / R) * (N / Cn), THREADS, SMEM, st>>>(m, N, cf, status, out, ux_out,
+                                                                 uy_out, phi_out);
     return true;
 }
 
@@ -1557,9 +1585,8 @@ template <typename T>
 void launch_leapfrog(const EventGeom *d_ev, int N, const State<T> &s,
                      C<T> *ux_out, C<T> *uy_out, T *phi_out,
                      const StepCoef<T> &cf, bool reunit, cudaStream_t st, double *status) {
-    // FP64 runs one thread per site: at 512^2 it takes 97 us a step against
-    // 108 us for the direction split (both FP64-pipe and latency bound at one
-    // 256-thread block per SM). FP32 runs both directions of a site in the
+    // FP64 runs two threads per site from shared-memory tiles filled by TMA
+    // (k_leapfrog_tile64), or one thread per site from plain loads. FP32 runs both directions of a site in the
     // two lanes of packed FP32 instructions, from shared-memory tiles filled
     // by TMA (k_leapfrog_tile) or from plain loads (k_leapfrog_pair).
     if constexpr (sizeof(T) == 4) {
@@ -1576,7 +1603,7 @@ void launch_leapfrog(const EventGeom *d_ev, int N, const State<T> &s,
     }
     if constexpr (sizeof(T) == 8) {
         if (N >= 32 && !reunit && use_tile64_kernel() &&
-            launch_leapfrog_tile64(N, s, ux_out, uy_out, phi_out, cf, status, st))
+            launch_leapfrog_tile64(N, s, s, s, ux_out, uy_out, phi_out, cf, status, st))
             return;
     }
     launch_leapfrog_site(d_ev, N, s, ux_out, uy_out, phi_out, cf, reunit, st);
@@ -1599,24 +1626,7 @@ void launch_leapfrog_into(const EventGeom *d_ev, int N, const State<double> &in,
     s.e2 = out.e2;
     s.pi = out.pi;
     if (!copy_e) {
-        using namespace tile64;
-        const uint64_t nn = (uint64_t)N;
-        const auto U64 = CU_TENSOR_MAP_DATA_TYPE_UINT64;
-        LoadMaps m;
-        const bool ok =
-            encode_tiled_3d(&m.ux, in.ux, U64, 8, 2 * nn, nn, 9, 2 * UC, UR, 9) &&
-            encode_tiled_3d(&m.uy, in.uy, U64, 8, 2 * nn, nn, 9, 2 * UC, UR, 9) &&
-            encode_tiled_3d(&m.phi, in.phi, U64, 8, nn, nn, 9, PC, PR, 9) &&
-            encode_tiled_3d(&m.e1, in.e1, U64, 8, nn, nn, 8, Cn, R, 8) &&
-            encode_tiled_3d(&m.e2, in.e2, U64, 8, nn, nn, 8, Cn, R, 8) &&
-            encode_tiled_3d(&m.pi, in.pi, U64, 8, nn, nn, 9, Cn, R, 9);
-        if (ok) {
-            cudaFuncSetAttribute(k_leapfrog_tile64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 SMEM);
-            k_leapfrog_tile64<<<(N / R) * (N / Cn), 128, SMEM, st>>>(m, N, cf, nullptr, s, out.ux,
-                                                                       out.uy, out.phi);
-            return;
-        }
+        if (launch_leapfrog_tile64(N, in, in, s, out.ux, out.uy, out.phi, cf, nullptr, st)) return;
         cudaMemcpyAsync(out.e1, in.e1, 8 * n * sizeof(double), cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(out.e2, in.e2, 8 * n * sizeof(double), cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(out.pi, in.pi, 9 * n * sizeof(double), cudaMemcpyDeviceToDevice, st);
@@ -1658,28 +1668,13 @@ void launch_inverse_se(int N, const State<T> &nxt, const State<T> &cur, const St
     const size_t n = (size_t)N * N;
     if constexpr (sizeof(T) == 8) {
         if (cf.do_pe && N >= 32 && use_tile64_kernel()) {
-            using namespace tile64;
-            const uint64_t nn = (uint64_t)N;
-            const auto U64 = CU_TENSOR_MAP_DATA_TYPE_UINT64;
-            LoadMaps m;
-            const bool ok =
-                encode_tiled_3d(&m.ux, cur.ux, U64, 8, 2 * nn, nn, 9, 2 * UC, UR, 9) &&
-                encode_tiled_3d(&m.uy, cur.uy, U64, 8, 2 * nn, nn, 9, 2 * UC, UR, 9) &&
-                encode_tiled_3d(&m.phi, cur.phi, U64, 8, nn, nn, 9, PC, PR, 9) &&
-                encode_tiled_3d(&m.e1, nxt.e1, U64, 8, nn, nn, 8, Cn, R, 8) &&
-                encode_tiled_3d(&m.e2, nxt.e2, U64, 8, nn, nn, 8, Cn, R, 8) &&
-                encode_tiled_3d(&m.pi, nxt.pi, U64, 8, nn, nn, 9, Cn, R, 9);
-            if (ok) {
-                StepCoef<double> rc = cf;
-                rc.dt_pe = -cf.dt_pe;
-                rc.do_pu = 0;
-                set_derived(rc);
-                cudaFuncSetAttribute(k_leapfrog_tile64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     SMEM);
-                k_leapfrog_tile64<<<(N / R) * (N / Cn), 128, SMEM, st>>>(m, N, rc, nullptr, cur,
-                                                                           nullptr, nullptr, nullptr);
+            StepCoef<double> rc = cf;
+            rc.dt_pe = -cf.dt_pe;
+            rc.do_pu = 0;
+            set_derived(rc);
+            if (launch_leapfrog_tile64(N, cur, nxt, cur, nullptr, nullptr, nullptr, rc, nullptr,
+                                       st))
                 return;
-            }
         }
     }
     k_inv_se<T><<<dim3((unsigned)((n + 127) / 128), 3), 128, 0, st>>>(N, nxt, cur, cf);

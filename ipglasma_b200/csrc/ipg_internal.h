@@ -75,7 +75,7 @@ struct LoadMaps {
     CUtensorMap ux, uy, phi, e1, e2, pi;
 };
 // the maps of the TMA tile kernels of precision T (FP32: 8 x 32 tiles, FP64:
-// 4 x 32 tiles) for a lattice of N x N sites with the given field planes;
+// 2 x 32 tiles) for a lattice of N x N sites with the given field planes;
 // false if the driver rejects them
 template <typename T>
 bool encode_step_maps(int N, const State<T> &s, LoadMaps *out);
