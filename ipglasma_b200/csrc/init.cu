@@ -122,6 +122,8 @@ __device__ __forceinline__ void restart_alpha(double alpha[8], uint64_t key,
 constexpr int kNewtonThreads = 128;
 // doubles of shared memory per thread: J (64), F, dalpha, alpha, best alpha
 constexpr int kNewtonSmem = 64 + 4 * 8;
+constexpr int kNewtonFirst = 8 * 18;  // doubles per block: the first Jacobian's exponentials
+constexpr double kFirstStep = 0.001;  // the difference step at alpha = 0 (Init.cpp:3380-3470)
 
 // the exponent held in shared memory, into registers, entry b replaced by v
 __device__ __forceinline__ void load_alpha(const double *al, int js, double out[8], int b = -1,
@@ -138,6 +140,34 @@ __device__ __forceinline__ void im_trace_ta(const M3<double> &m, double out[8]) 
     for (int a = 0; a < 8; a++) out[a] = t[a].i;
 }
 
+// What the iteration needs of a link at the exponent alpha:
+// U = exp(i alpha.t) U0, U0 = U1 U2, S = U1 + U2. Daggers are taken inside the
+// products (mul_nd: A B^dag).
+struct Link {
+    M3<double> U0, S, U;
+    __device__ __forceinline__ Link(const M3<double> &U1, const M3<double> &U2) {
+        U0 = mul(U1, U2);
+        S = U1;
+        add_to(S, U2);
+    }
+    __device__ __forceinline__ void set(const double a8[8]) { U = mul(exp_from_coeff(a8), U0); }
+    __device__ __forceinline__ void start() { U = U0; }  // alpha = 0
+    // Im tr(t^a (S - S^dag))
+    __device__ __forceinline__ void constant(double out[8]) const {
+        im_trace_ta(minus(S, dagger(S)), out);
+    }
+    // Im tr(t^a (S U^dag - U S^dag))
+    __device__ __forceinline__ void residual(double out[8]) const {
+        M3<double> Mt = mul_nd(S, U);
+        sub_from(Mt, mul_nd(U, S));
+        im_trace_ta(Mt, out);
+    }
+    // Im tr(t^a S (E1 U0 - U)^dag)
+    __device__ __forceinline__ void difference(const M3<double> &E1, double out[8]) const {
+        im_trace_ta(mul_nd(S, minus(mul(E1, U0), U)), out);
+    }
+};
+
 __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
     // this thread's slice of shared memory, element k at base[k * js]
     extern __shared__ double newton_j[];
@@ -146,34 +176,40 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
     double *Fa = J + 64 * js, *dalpha = J + 72 * js, *al = J + 80 * js, *best_al = J + 88 * js;
     const size_t n = (size_t)A.N * A.N;
     const size_t lid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (lid >= 2 * n) return;
-    if (A.redo_only && A.status[lid] != -1) return;
+    const bool mine = lid < 2 * n && !(A.redo_only && A.status[lid] != -1);
+    // The iteration starts at alpha = 0, where the differenced exponentials of
+    // the first Jacobian are exp(i 0.001 t^b) for every link: eight threads
+    // evaluate them for the block (nine of a link's exponentials saved; a link
+    // takes three or four iterations)
+    double *first = newton_j + kNewtonSmem * js;
+    if (!__syncthreads_or(mine)) return;
+    if (threadIdx.x < 8) {
+        double q[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) q[k] = k == (int)threadIdx.x ? kFirstStep : 0.;
+        const M3<double> e = exp_from_coeff(q);
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            first[18 * threadIdx.x + 2 * k] = e.m[k].r;
+            first[18 * threadIdx.x + 2 * k + 1] = e.m[k].i;
+        }
+    }
+    __syncthreads();
+    if (!mine) return;
     // link order of the reference loop: per site, x then y (Init.cpp:2498-2516)
     const size_t pos = lid >> 1;
     const int dir = (int)(lid & 1);
-    // Daggers of S and of the iterate are taken inside the products
-    // (mul_nd: A B^dag), the best iterate is kept as its exponent, and the
-    // small arrays the iteration indexes by data sit in shared memory: that
-    // keeps the live state in registers. The iterates are bit-identical to
-    // forming the daggers and the best matrix.
-    M3<double> U0, S;
-    {
-        const M3<double> U1 = ld_m3(dir ? A.u1y : A.u1x, pos, n);
-        const M3<double> U2 = ld_m3(dir ? A.u2y : A.u2x, pos, n);
-        U0 = mul(U1, U2);
-        S = U1;
-        add_to(S, U2);
-    }
-    double traceCache[8];  // Im tr(t^a (S - S^dag))
-    im_trace_ta(minus(S, dagger(S)), traceCache);
+    const C<double> *u1 = dir ? A.u1y : A.u1x, *u2 = dir ? A.u2y : A.u2x;
+    // The best iterate is kept as its exponent, and the small arrays the
+    // iteration indexes by data sit in shared memory: that keeps the live state
+    // in registers.
+    Link L(ld_m3(u1, pos, n), ld_m3(u2, pos, n));
+    double traceCache[8];
+    L.constant(traceCache);
 
     double a8[8];
 #pragma unroll
-    for (int a = 0; a < 8; a++) {
-        al[a * js] = 0.;
-        a8[a] = 0.;
-    }
-    M3<double> Usol = mul(exp_from_coeff(a8), U0);
+    for (int a = 0; a < 8; a++) al[a * js] = 0.;
     bool have_best = false;  // false stands for the identity
     double Fzero = 10., FzeroMin = 1e6;
     int iter = 0, nRestart = 0, total = 0;
@@ -181,12 +217,17 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
     while (Fzero > 1e-6 && iter < A.max_iter && nRestart < A.max_restart) {
         iter++;
         total++;
+        // U at the current exponent
+        if (total == 1) {
+            L.start();
+        } else {
+            load_alpha(al, js, a8);
+            L.set(a8);
+        }
         Fzero = 0.;
         {
-            M3<double> Mt = mul_nd(S, Usol);
-            sub_from(Mt, mul_nd(Usol, S));
             double tl[8];
-            im_trace_ta(Mt, tl);
+            L.residual(tl);
 #pragma unroll
             for (int a = 0; a < 8; a++) {
                 // -(traceCache + traceLoc), imaginary part
@@ -198,12 +239,19 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
         bool good = true;
         for (int b = 0; b < 8; b++) {
             const double ab = al[b * js];
-            const double d = fmax(0.001, fmin(10., 0.01 * fabs(ab)));
+            const double d = fmax(kFirstStep, fmin(10., 0.01 * fabs(ab)));
             const double ap = ab + d;
-            load_alpha(al, js, a8, b, ap);
-            const M3<double> Mt = mul_nd(S, minus(mul(exp_from_coeff(a8), U0), Usol));
+            M3<double> E1;
+            if (total == 1) {
+#pragma unroll
+                for (int k = 0; k < 9; k++)
+                    E1.m[k] = {first[18 * b + 2 * k], first[18 * b + 2 * k + 1]};
+            } else {
+                load_alpha(al, js, a8, b, ap);
+                E1 = exp_from_coeff(a8);
+            }
             double tl[8];
-            im_trace_ta(Mt, tl);
+            L.difference(E1, tl);
             double mcheck = 0.;
 #pragma unroll
             for (int a = 0; a < 8; a++) {
@@ -217,11 +265,11 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
         }
         if (!good) {
             // analytic approximation (Init.cpp:3419-3431)
-            const M3<double> Usold = dagger(Usol);
+            const M3<double> Usold = dagger(L.U);
             for (int b = 0; b < 8; b++) {
                 const M3<double> Mt = ta_mul(b, Usold);
                 for (int a = 0; a < 8; a++) {
-                    const M3<double> Ma = ta_mul(a, S);
+                    const M3<double> Ma = ta_mul(a, L.S);
                     J[(a * 8 + b) * js] = -2. * re_trace_mul(Ma, Mt);
                 }
             }
@@ -241,82 +289,99 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
 #pragma unroll
             for (int a = 0; a < 8; a++) al[a * js] = a8[a];
         }
-        load_alpha(al, js, a8);
-        Usol = mul(exp_from_coeff(a8), U0);
         if (Fzero < FzeroMin) {
             FzeroMin = Fzero;
             have_best = true;
 #pragma unroll
-            for (int a = 0; a < 8; a++) best_al[a * js] = a8[a];
+            for (int a = 0; a < 8; a++) best_al[a * js] = al[a * js];
         }
         if (iter == A.max_iter) {
             restart_alpha(a8, A.philox_key, (uint32_t)lid, draws++);
 #pragma unroll
             for (int a = 0; a < 8; a++) al[a * js] = a8[a];
-            Usol = mul(exp_from_coeff(a8), U0);
             nRestart++;
             iter = 0;
         }
     }
     int status = draws ? 1 : 0;
-    if (nRestart == A.max_restart) {
-        if (have_best) {
-            load_alpha(best_al, js, a8);
-            Usol = mul(exp_from_coeff(a8), U0);
-        } else {
-            set_identity(Usol);
-        }
-        status = 2;
-    } else if (A.tol < 1e-6) {
-        // polish beyond the reference's criterion (for derivatives through the
-        // root): Newton steps with a central-difference Jacobian, no restarts,
-        // keeping the iterate with the smallest residual
-        double bestF = 1e300;
-        for (int p = 0; p < 8; p++) {
-            double s = 0.;
-            {
-                M3<double> Mt = mul_nd(S, Usol);
-                sub_from(Mt, mul_nd(Usol, S));
-                double tl[8];
-                im_trace_ta(Mt, tl);
-                for (int a = 0; a < 8; a++) {
-                    const double f = -(traceCache[a] + tl[a]);
-                    Fa[a * js] = f;
-                    s += fabs(f);
-                }
-            }
-            if (s < bestF) {
-                bestF = s;
-                for (int a = 0; a < 8; a++) best_al[a * js] = al[a * js];
-            }
-            if (s < A.tol) break;
-            for (int b = 0; b < 8; b++) {
-                const double h = 1e-6, a0 = al[b * js];
-                load_alpha(al, js, a8, b, a0 + h);
-                const M3<double> Up = mul(exp_from_coeff(a8), U0);
-                load_alpha(al, js, a8, b, a0 - h);
-                const M3<double> Um = mul(exp_from_coeff(a8), U0);
-                const M3<double> dU = scaled(minus(Up, Um), 0.5 / h);
-                M3<double> Mt = mul_nd(S, dU);
-                sub_from(Mt, mul_nd(dU, S));
-                double tl[8];
-                im_trace_ta(Mt, tl);
-                for (int a = 0; a < 8; a++) J[(a * 8 + b) * js] = -tl[a];
-            }
-            lu_solve8(J, Fa, dalpha, js);
-            for (int a = 0; a < 8; a++) al[a * js] -= dalpha[a * js];
-            load_alpha(al, js, a8);
-            Usol = mul(exp_from_coeff(a8), U0);
-        }
-        for (int a = 0; a < 8; a++) al[a * js] = best_al[a * js];
-        load_alpha(al, js, a8);
-        Usol = mul(exp_from_coeff(a8), U0);
+    const bool failed = nRestart == A.max_restart;
+    if (failed) status = 2;
+    if (failed && !have_best) {
+        set_identity(L.U);
+    } else {
+        load_alpha(failed ? best_al : al, js, a8);
+        L.set(a8);
     }
-    st_m3(dir ? A.uy : A.ux, pos, n, Usol);
+    st_m3(dir ? A.uy : A.ux, pos, n, L.U);
     if (A.alpha)
         for (int a = 0; a < 8; a++) A.alpha[(size_t)a * 2 * n + lid] = al[a * js];
     A.iters[lid] = total;
     A.status[lid] = status;
+}
+
+// Beyond the reference's criterion (for derivatives through the root): Newton
+// steps from k_newton's exponent with a central-difference Jacobian, no
+// restarts, keeping the iterate with the smallest residual. A kernel of its
+// own, so that its exponentials cost k_newton no registers.
+__global__ void __launch_bounds__(kNewtonThreads) k_newton_polish(NewtonArgs A) {
+    extern __shared__ double newton_j[];
+    constexpr int js = kNewtonThreads;
+    double *J = newton_j + threadIdx.x;
+    double *Fa = J + 64 * js, *dalpha = J + 72 * js, *al = J + 80 * js, *best_al = J + 88 * js;
+    const size_t n = (size_t)A.N * A.N;
+    const size_t lid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (lid >= 2 * n || A.status[lid] == 2) return;
+    const size_t pos = lid >> 1;
+    const int dir = (int)(lid & 1);
+    const C<double> *u1 = dir ? A.u1y : A.u1x, *u2 = dir ? A.u2y : A.u2x;
+    Link L(ld_m3(u1, pos, n), ld_m3(u2, pos, n));
+    double traceCache[8];
+    L.constant(traceCache);
+    double a8[8];
+    for (int a = 0; a < 8; a++) al[a * js] = A.alpha[(size_t)a * 2 * n + lid];
+    if (isnan(al[0])) return;  // a link that k_newton_fast took to the tolerance
+    double bestF = 1e300;
+    for (int p = 0; p < 8; p++) {
+        load_alpha(al, js, a8);
+        L.set(a8);
+        double s = 0.;
+        {
+            double tl[8];
+            L.residual(tl);
+            for (int a = 0; a < 8; a++) {
+                const double f = -(traceCache[a] + tl[a]);
+                Fa[a * js] = f;
+                s += fabs(f);
+            }
+        }
+        if (s < bestF) {
+            bestF = s;
+            for (int a = 0; a < 8; a++) best_al[a * js] = al[a * js];
+        }
+        if (s < A.tol) break;
+        for (int b = 0; b < 8; b++) {
+            const double h = 1e-6, a0 = al[b * js];
+            load_alpha(al, js, a8, b, a0 + h);
+            const M3<double> Up = mul(exp_from_coeff(a8), L.U0);
+            load_alpha(al, js, a8, b, a0 - h);
+            const M3<double> Um = mul(exp_from_coeff(a8), L.U0);
+            const M3<double> dU = scaled(minus(Up, Um), 0.5 / h);
+            M3<double> Mt = mul_nd(L.S, dU);
+            sub_from(Mt, mul_nd(dU, L.S));
+            double tl[8];
+            im_trace_ta(Mt, tl);
+            for (int a = 0; a < 8; a++) J[(a * 8 + b) * js] = -tl[a];
+        }
+        lu_solve8(J, Fa, dalpha, js);
+        for (int a = 0; a < 8; a++) al[a * js] -= dalpha[a * js];
+    }
+    // no finite residual at all: the exponent stays as the reference's
+    // iteration left it
+    if (!(bestF < 1e300)) return;
+    load_alpha(best_al, js, a8);
+    L.set(a8);
+    st_m3(dir ? A.uy : A.ux, pos, n, L.U);
+    for (int a = 0; a < 8; a++) A.alpha[(size_t)a * 2 * n + lid] = best_al[a * js];
 }
 
 // ---------------------------------------------------------------------------
@@ -407,7 +472,9 @@ __global__ void __launch_bounds__(kFastThreads) k_newton_fast(NewtonArgs A) {
 
 void launch_newton(const NewtonArgs &a, cudaStream_t st) {
     const size_t links = 2 * (size_t)a.N * a.N;
-    const size_t smem = sizeof(double) * kNewtonSmem * kNewtonThreads;  // 96 KB
+    const unsigned blocks = (unsigned)((links + kNewtonThreads - 1) / kNewtonThreads);
+    // 97 KB: two blocks an SM
+    const size_t smem = sizeof(double) * (kNewtonSmem * kNewtonThreads + kNewtonFirst);
     cudaFuncSetAttribute(k_newton, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     NewtonArgs b = a;
     if (a.mode == 1) {
@@ -418,8 +485,12 @@ void launch_newton(const NewtonArgs &a, cudaStream_t st) {
                         fsmem, st>>>(a);
         b.redo_only = 1;
     }
-    k_newton<<<(unsigned)((links + kNewtonThreads - 1) / kNewtonThreads), kNewtonThreads, smem,
-               st>>>(b);
+    k_newton<<<blocks, kNewtonThreads, smem, st>>>(b);
+    if (a.tol < 1e-6) {
+        cudaFuncSetAttribute(k_newton_polish, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
+        k_newton_polish<<<blocks, kNewtonThreads, smem, st>>>(b);
+    }
 }
 
 // ---------------------------------------------------------------------------
