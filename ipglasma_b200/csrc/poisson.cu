@@ -164,12 +164,33 @@ template <int LOGN>
 constexpr int col_threads() {
     return cols_per_block<LOGN>() * ((1 << LOGN) / 8);
 }
-// sequence stride of the forward row kernel: there lanes 2i and 2i+1 hold the
-// same points of neighbouring sequences (channels 2h, 2h+1), so the stride is
-// made 4 mod 8 (in 16-byte units) to put the pair half a bank cycle apart;
-// with fft_seq_stride (1 mod 8) lane 2i+1 met lane 2i+2 on the same banks
+// Sequence strides in shared memory, in complex elements. One wavefront
+// serves BANKS = 8 (double) or 16 (float) lanes; a sequence's own accesses
+// (consecutive points, or 9 t in the first pass's stores) fall on different
+// banks by fft_pad, and the stride has to keep the lanes of neighbouring
+// sequences apart from them. Wavefronts of the column kernel hold JB columns
+// at BANKS / JB points: the stride is BANKS / JB modulo BANKS. Lanes 2i and
+// 2i+1 of the forward row kernel hold the same points of neighbouring
+// sequences: BANKS / 2 modulo BANKS. (With N + N/8 + 1 for every kernel, four
+// lanes met on a bank in the FP32 columns at 1024^2 and two at 512^2.)
+template <typename R>
+constexpr int smem_banks() {
+    return sizeof(R) == 8 ? 8 : 16;
+}
+template <typename R>
+constexpr int stride_at(int N, int want) {
+    int s = N + (N >> 3);
+    while (s % smem_banks<R>() != want % smem_banks<R>()) s++;
+    return s;
+}
+template <int LOGN, typename R>
+constexpr int col_stride() {
+    constexpr int jb = cols_per_block<LOGN>();
+    return stride_at<R>(1 << LOGN, jb < smem_banks<R>() ? smem_banks<R>() / jb : 1);
+}
+template <typename R>
 constexpr int fwd_seq_stride(int N) {
-    return fft_seq_stride(N) + ((12 - fft_seq_stride(N) % 8) % 8);
+    return stride_at<R>(N, smem_banks<R>() / 2);
 }
 
 }  // namespace
@@ -178,7 +199,7 @@ template <int LOGN, typename R>
 __global__ void __launch_bounds__(row_threads<LOGN>()) k_rows_fwd(WilsonArgs w, int k0) {
     if (w.skip && *w.skip) return;
     constexpr int N = 1 << LOGN, TPS = N / 8, RPB = rows_per_block<LOGN>();
-    constexpr int S = fwd_seq_stride(N);
+    constexpr int S = fwd_seq_stride<R>(N);
     extern __shared__ __align__(16) unsigned char smraw[];
     C<R> *sm = reinterpret_cast<C<R> *>(smraw);
     const size_t n = (size_t)N * N;
@@ -255,7 +276,7 @@ template <int LOGN, bool CONV = true, typename R = double>
 __global__ void __launch_bounds__(col_threads<LOGN>(), 2) k_cols(WilsonArgs w) {
     if (w.skip && *w.skip) return;
     constexpr int N = 1 << LOGN, TPS = N / 8, JB = cols_per_block<LOGN>();
-    constexpr int S = fft_seq_stride(N);
+    constexpr int S = col_stride<LOGN, R>();
     extern __shared__ __align__(16) unsigned char smraw[];
     C<R> *sm = reinterpret_cast<C<R> *>(smraw);
     const size_t n = (size_t)N * N;
@@ -354,8 +375,8 @@ static void launch_sheets_t(const WilsonArgs &w, int k0, int ns, cudaStream_t st
     constexpr int N = 1 << LOGN;
     constexpr int RPB = rows_per_block<LOGN>(), JB = cols_per_block<LOGN>();
     const size_t row_smem = sizeof(C<R>) * RPB * 4 * fft_seq_stride(N);
-    const size_t fwd_smem = sizeof(C<R>) * RPB * 4 * fwd_seq_stride(N);
-    const size_t col_smem = sizeof(C<R>) * JB * fft_seq_stride(N);
+    const size_t fwd_smem = sizeof(C<R>) * RPB * 4 * fwd_seq_stride<R>(N);
+    const size_t col_smem = sizeof(C<R>) * JB * col_stride<LOGN, R>();
     // the attribute is per device: set it on every launch (a host-side call
     // without a device round trip)
     cudaFuncSetAttribute(k_rows_fwd<LOGN, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -384,8 +405,8 @@ template <int LOGN>
 static void launch_forward(const WilsonArgs &w, int ns, cudaStream_t st) {
     constexpr int N = 1 << LOGN;
     constexpr int RPB = rows_per_block<LOGN>(), JB = cols_per_block<LOGN>();
-    const size_t fwd_smem = sizeof(double2) * RPB * 4 * fwd_seq_stride(N);
-    const size_t col_smem = sizeof(double2) * JB * fft_seq_stride(N);
+    const size_t fwd_smem = sizeof(double2) * RPB * 4 * fwd_seq_stride<double>(N);
+    const size_t col_smem = sizeof(double2) * JB * col_stride<LOGN, double>();
     cudaFuncSetAttribute(k_rows_fwd<LOGN, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)fwd_smem);
     cudaFuncSetAttribute(k_cols<LOGN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
