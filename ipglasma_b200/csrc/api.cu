@@ -1710,6 +1710,7 @@ ipg_status ipg_get_field(ipg_ctx *c, int which, double *out) {
     const size_t n = c->n;
     if (which == IPG_VA || which == IPG_VB || which == IPG_UX || which == IPG_UY) {
         if (which == IPG_UX || which == IPG_UY) IPG_TRY(state64(c));
+        IPG_TRY(sync(c));  // the copies below are not on the context's stream
         const C<double> *src = which == IPG_VA ? c->VA
                                : which == IPG_VB ? c->VB
                                : which == IPG_UX ? c->s64.ux
@@ -1721,6 +1722,7 @@ ipg_status ipg_get_field(ipg_ctx *c, int which, double *out) {
         return IPG_OK;
     }
     IPG_TRY(state64(c));
+    IPG_TRY(sync(c));
     const bool tl = (which == IPG_E1 || which == IPG_E2);
     const double *src = which == IPG_E1 ? c->s64.e1
                         : which == IPG_E2 ? c->s64.e2
