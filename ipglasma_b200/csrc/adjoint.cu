@@ -929,60 +929,74 @@ __global__ void k_adj_link_products(int N, const C<double> *VA, const C<double> 
     }
 }
 
-// one sheet of V_k = exp(-i A_k.t) V_{k-1}, backwards: V <- V_{k-1} (time
-// reversal by the unitary inverse), V_bar <- V_bar_{k-1}, and the packed A
-// of the sheet in work is replaced by its adjoint A_bar
-__global__ void __launch_bounds__(128) k_adj_wilson_sheet(int N, double2 *work, C<double> *V,
-                                                          C<double> *Vb) {
+// The sheets of a batch of V_k = exp(-i A_k.t) V_{k-1}, backwards: V <-
+// V_{k-1} (time reversal by the unitary inverse), V_bar <- V_bar_{k-1}, and
+// the packed A of each sheet in work is replaced by its adjoint A_bar. The
+// recursion is local to a site, so one launch takes all sheets of a batch, V
+// and V_bar staying in the thread's registers (a launch a sheet took 9 us at
+// 128^2 and 19 us at 256^2).
+__global__ void __launch_bounds__(128) k_adj_wilson_sheets(int N, int ns, double2 *work,
+                                                           C<double> *V, C<double> *Vb) {
     const size_t n = (size_t)N * N;
     const size_t pos = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= n) return;
-    double q[8];
-    for (int c = 0; c < 4; c++) {
-        const double2 v = work[(size_t)c * n + pos];
-        q[2 * c] = -v.x;
-        q[2 * c + 1] = -v.y;
+    Md Vk = ld_m3(V, pos, n), Vbk = ld_adj(Vb, pos, n);
+    for (int s = ns - 1; s >= 0; s--) {
+        double2 *w = work + (size_t)s * 4 * n + pos;
+        double q[8];
+        for (int c = 0; c < 4; c++) {
+            const double2 v = w[(size_t)c * n];
+            q[2 * c] = -v.x;
+            q[2 * c + 1] = -v.y;
+        }
+        const Md e = exp_from_coeff(q);
+        Vk = mul_dn(e, Vk);
+        const Md eb = mul_nd(Vbk, Vk);
+        Vbk = mul_dn(e, Vbk);
+        double qb[8];
+        if (!exp_vjp(q, eb, qb))
+            for (int b = 0; b < 8; b++) qb[b] = re_dot(eb, dexp(q, b, kDexpStep));
+        for (int c = 0; c < 4; c++)
+            w[(size_t)c * n] = make_double2(-qb[2 * c], -qb[2 * c + 1]);
     }
-    const Md e = exp_from_coeff(q);
-    const Md Vk = ld_m3(V, pos, n), Vbk = ld_adj(Vb, pos, n);
-    const Md Vprev = mul_dn(e, Vk);
-    const Md eb = mul_nd(Vbk, Vprev);
-    st_m3(V, pos, n, Vprev);
-    st_adj(Vb, pos, n, mul_dn(e, Vbk));
-    double qb[8];
-    if (!exp_vjp(q, eb, qb))
-        for (int b = 0; b < 8; b++) qb[b] = re_dot(eb, dexp(q, b, kDexpStep));
-    for (int c = 0; c < 4; c++) work[(size_t)c * n + pos] = make_double2(-qb[2 * c], -qb[2 * c + 1]);
+    st_m3(V, pos, n, Vk);
+    st_adj(Vb, pos, n, Vbk);
 }
 
-// rho = g sqrt(g2mu2 / Ny) xi: the packed rho_bar of one sheet in work ->
-// g2mu2_bar (accumulated) and, if rho_out is set, rho_bar as [n][8]
+// rho = g sqrt(g2mu2 / Ny) xi: the packed rho_bar of sheets k0 .. k0+ns-1 in
+// work -> g2mu2_bar (accumulated, sheets from the top) and, if rho_out is set,
+// rho_bar as [ns][n][8] (rho_out at sheet k0). One launch a batch.
 __global__ void k_adj_rho(int N, int Ny, double g, const double *g2mu2, const double *xi,
-                          uint64_t key, uint32_t nucleus, int k, const double2 *work,
+                          uint64_t key, uint32_t nucleus, int k0, int ns, const double2 *work,
                           double *g2mu_bar, double *rho_out) {
     const size_t n = (size_t)N * N;
     const size_t pos = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (pos >= n) return;
-    double z[8];
-    if (xi) {
-        for (int a = 0; a < 8; a++) z[a] = xi[((size_t)k * n + pos) * 8 + a];
-    } else {
-        for (int h = 0; h < 2; h++)
-            for (int p = 0; p < 2; p++)
-                normal2({(uint32_t)pos, (uint32_t)k, (nucleus << 1) | (uint32_t)h, 0u}, key, p,
-                        z + 4 * h + 2 * p);
-    }
-    double acc = 0.;
-    for (int c = 0; c < 4; c++) {
-        const double2 v = work[(size_t)c * n + pos];
-        acc += v.x * z[2 * c] + v.y * z[2 * c + 1];
-        if (rho_out) {
-            rho_out[pos * 8 + 2 * c] = v.x;
-            rho_out[pos * 8 + 2 * c + 1] = v.y;
-        }
-    }
     const double m = g2mu2[pos];
-    if (m > 0.) g2mu_bar[pos] += acc * g / (2. * sqrt(m * Ny));
+    double bar = g2mu_bar[pos];
+    for (int s = ns - 1; s >= 0; s--) {
+        const int k = k0 + s;
+        double z[8];
+        if (xi) {
+#pragma unroll
+            for (int a = 0; a < 8; a++) z[a] = xi[((size_t)k * n + pos) * 8 + a];
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                normal4({(uint32_t)pos, (uint32_t)k, (nucleus << 1) | (uint32_t)h, 0u}, key,
+                        z + 4 * h);
+        }
+        double acc = 0.;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const double2 v = work[((size_t)s * 4 + c) * n + pos];
+            acc += v.x * z[2 * c] + v.y * z[2 * c + 1];
+            if (rho_out)
+                reinterpret_cast<double2 *>(rho_out)[((size_t)s * n + pos) * 4 + c] = v;
+        }
+        if (m > 0.) bar += acc * g / (2. * sqrt(m * Ny));
+    }
+    g2mu_bar[pos] = bar;
 }
 
 // ---------------------------------------------------------------------------
@@ -1105,17 +1119,17 @@ void launch_adjoint_init_links(const AdjInitArgs &A, cudaStream_t st) {
                                                    A.vbA, A.vbB);
 }
 
-void launch_adjoint_wilson_sheet(int N, double2 *work, C<double> *V, C<double> *Vb,
-                                 cudaStream_t st) {
+void launch_adjoint_wilson_sheets(int N, int ns, double2 *work, C<double> *V, C<double> *Vb,
+                                  cudaStream_t st) {
     const size_t n = (size_t)N * N;
-    k_adj_wilson_sheet<<<blocks(n), 128, 0, st>>>(N, work, V, Vb);
+    k_adj_wilson_sheets<<<blocks(n), 128, 0, st>>>(N, ns, work, V, Vb);
 }
 
-void launch_adjoint_rho(const WilsonArgs &w, int k, double *g2mu_bar, double *rho_out,
+void launch_adjoint_rho(const WilsonArgs &w, int k0, int ns, double *g2mu_bar, double *rho_out,
                         cudaStream_t st) {
     const size_t n = (size_t)w.N * w.N;
     k_adj_rho<<<blocks(n), 128, 0, st>>>(w.N, w.Ny, w.g, w.g2mu2, w.xi, w.philox_key, w.nucleus,
-                                         k, w.work, g2mu_bar, rho_out);
+                                         k0, ns, w.work, g2mu_bar, rho_out);
 }
 
 }  // namespace ipg

@@ -1879,32 +1879,26 @@ ipg_status backward_inputs(ipg_ctx *c, double *grad_g2mu, double *grad_rho) {
         launch_wilson_amp(w, st);
         IPG_LAUNCHED(c, 1);
         // batches of work_sheets sheets from the top: the transforms of a
-        // batch (A_k, then the Poisson map of A_bar_k) run as one launch each,
-        // the product recursion and the rho adjoint sheet by sheet in the
-        // order k = Ny-1 .. 0 (the accumulation order of g2mu_bar)
+        // batch (A_k, then the Poisson map of A_bar_k), the product recursion
+        // and the rho adjoint run as one launch each, sheets in the order
+        // k = Ny-1 .. 0 (the accumulation order of g2mu_bar)
         const int S = c->work_sheets;
         for (int kb = Ny; kb > 0; kb -= S) {
             const int k0 = std::max(0, kb - S), ns = kb - k0;
             w.rho_in = nullptr;
             launch_wilson_sheets(w, k0, ns, st);  // slot k - k0 = A_k
             IPG_LAUNCHED(c, 3);
-            for (int k = kb - 1; k >= k0; k--) {
-                // slot k - k0 becomes A_bar_k
-                launch_adjoint_wilson_sheet(N, work + (size_t)(k - k0) * 4 * n, vcur, vb, st);
-                IPG_LAUNCHED(c, 1);
-            }
+            // slot k - k0 becomes A_bar_k, sheets from the top
+            launch_adjoint_wilson_sheets(N, ns, work, vcur, vb, st);
+            IPG_LAUNCHED(c, 1);
             w.rho_in = work;
             launch_poisson_sheets(w, ns, st);  // in place: slot k - k0 = rho_bar_k
             IPG_LAUNCHED(c, 3);
             w.rho_in = nullptr;
-            for (int k = kb - 1; k >= k0; k--) {
-                WilsonArgs ws = w;
-                ws.work = work + (size_t)(k - k0) * 4 * n;
-                launch_adjoint_rho(ws, k, A.g2mu_bar + nuc * n,
-                                   grad_rho ? A.rho_all + ((size_t)nuc * Ny + k) * n * 8 : nullptr,
-                                   st);
-                IPG_LAUNCHED(c, 1);
-            }
+            launch_adjoint_rho(w, k0, ns, A.g2mu_bar + nuc * n,
+                               grad_rho ? A.rho_all + ((size_t)nuc * Ny + k0) * n * 8 : nullptr,
+                               st);
+            IPG_LAUNCHED(c, 1);
         }
     }
     IPG_CUDA(c, cudaEventRecord(c->ev_nuc_join, c->stream_v));

@@ -354,12 +354,13 @@ struct AdjInitArgs {
     C<double> *b1x, *b2x, *b1y, *b2y, *vbA, *vbB;
 };
 void launch_adjoint_init_links(const AdjInitArgs &a, cudaStream_t st);
-// one sheet backwards through V_k = exp(-i A_k.t) V_{k-1}; work holds the
-// packed A_k on entry and A_bar_k on return
-void launch_adjoint_wilson_sheet(int N, double2 *work, C<double> *V, C<double> *Vb,
-                                 cudaStream_t st);
-// packed rho_bar of sheet k in w.work -> g2mu2_bar (+=) and rho_bar [n][8]
-void launch_adjoint_rho(const WilsonArgs &w, int k, double *g2mu_bar, double *rho_out,
+// ns sheets backwards through V_k = exp(-i A_k.t) V_{k-1}, the last one
+// first; work holds their packed A_k on entry and A_bar_k on return
+void launch_adjoint_wilson_sheets(int N, int ns, double2 *work, C<double> *V, C<double> *Vb,
+                                  cudaStream_t st);
+// packed rho_bar of sheets k0 .. k0+ns-1 in w.work -> g2mu2_bar (+=, the last
+// sheet first) and rho_bar [ns][n][8]
+void launch_adjoint_rho(const WilsonArgs &w, int k0, int ns, double *g2mu_bar, double *rho_out,
                         cudaStream_t st);
 
 struct LandauArgs {
