@@ -62,7 +62,7 @@ struct ipg_ctx {
     // FP32 (the transforms of the FP32 form run in FP32)
     float2 *twiddle32 = nullptr;
     float *green32 = nullptr;
-    double *amp = nullptr;
+    double *amp = nullptr, *ampB = nullptr;  // charge amplitudes of A and B
     double2 *work = nullptr, *work2 = nullptr;
     double *nuc_xyz = nullptr, *nuc_gx = nullptr, *nuc_gy = nullptr;  // ipg_set_nuclei
     struct {  // ipg_set_nuclei_ipsat (allocated by its first call)
@@ -121,7 +121,6 @@ struct ipg_ctx {
         // initial-condition adjoint: U1/U2 adjoints, V adjoints, a V copy
         C<double> *b1x = nullptr, *b2x = nullptr, *b1y = nullptr, *b2y = nullptr;
         C<double> *vbA = nullptr, *vbB = nullptr, *vcur = nullptr, *vcur2 = nullptr;
-        double *amp2 = nullptr;  // nucleus B's rho amplitude in the input adjoint
         double *g2mu_bar = nullptr;
         double *rho_all = nullptr;  // [2][Ny][n][8] rho adjoint, kept on the device
         // FP32 adjoint (contexts of the FP32 form): the bulk form's own states
@@ -817,6 +816,7 @@ ipg_status ipg_create(const ipg_config *cfg, ipg_ctx **out) {
     IPG_TRY(dalloc(c, &c->twiddle, (size_t)N));
     IPG_TRY(dalloc(c, &c->green, n));
     IPG_TRY(dalloc(c, &c->amp, n));
+    IPG_TRY(dalloc(c, &c->ampB, n));
     // work buffer of a sheet batch: up to 128 MB (8 sheets at 512^2, 32 at
     // 256^2). Larger batches give each transform launch more parallelism:
     // the 512^2 Wilson-line stage takes 3.59 ms at 128 MB, 3.68 ms at 64 MB,
@@ -1251,11 +1251,26 @@ static ipg_status init_enqueue(ipg_ctx *c, bool from_wilson) {
     // scal[38]: set by a step kernel whose bounded wait gave up
     IPG_CUDA(c, cudaMemsetAsync(c->scal + 38, 0, sizeof(double), c->stream));
 
-    // Wilson lines, nucleus A then B (Init.cpp:1688-1847)
+    // Wilson lines, nucleus A then B (Init.cpp:1688-1847). Where the sheets of a
+    // nucleus are one batch (small lattices, whose kernels leave the GPU partly
+    // idle), B runs beside A: on stream_v, with the other work buffer and an
+    // amplitude array of its own (us for both nuclei's
+    // lines, 50 sheets, one after the other and side by side: FP64 64^2 232 ->
+    // 158, 128^2 341 -> 276, 256^2 (32 sheets) 640 -> 577; FP32 64^2 132 -> 107,
+    // 128^2 206 -> 172, 256^2 614 -> 588, 512^2 (16 sheets) 758 -> 728). Several
+    // batches a nucleus already run the products of one beside the transforms
+    // of the next.
+    const int sheets_a_batch = is_fp32(c) ? 2 * c->work_sheets : c->work_sheets;
+    const bool side_by_side = !from_wilson && c->cfg.Ny <= sheets_a_batch;
+    if (side_by_side) {
+        IPG_CUDA(c, cudaEventRecord(c->ev_nuc_fork, c->stream));
+        IPG_CUDA(c, cudaStreamWaitEvent(c->stream_v, c->ev_nuc_fork, 0));
+    }
     int batch = 0;
     for (int nuc = 0; nuc < (from_wilson ? 0 : 2); nuc++) {
         C<double> *V = nuc ? c->VB : c->VA;
-        k_identity<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(n, V);
+        cudaStream_t st = nuc && side_by_side ? c->stream_v : c->stream;
+        k_identity<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, V);
         IPG_LAUNCHED(c, 1);
         WilsonArgs w;
         w.N = N;
@@ -1268,16 +1283,22 @@ static ipg_status init_enqueue(ipg_ctx *c, bool from_wilson) {
         w.nucleus = (uint32_t)nuc;
         w.twiddle = c->twiddle;
         w.green = c->green;
-        w.amp = c->amp;
+        w.amp = nuc ? c->ampB : c->amp;
         w.work = c->work;
         w.V = V;
         // the FP32 form transforms in FP32: twice the sheets fit a work buffer
         w.fp32 = is_fp32(c) ? 1 : 0;
         w.twiddle32 = c->twiddle32;
         w.green32 = c->green32;
-        const int sheets = w.fp32 ? 2 * c->work_sheets : c->work_sheets;
-        launch_wilson_amp(w, c->stream);
+        const int sheets = sheets_a_batch;
+        launch_wilson_amp(w, st);
         IPG_LAUNCHED(c, 1);
+        if (side_by_side) {
+            w.work = nuc ? c->work2 : c->work;
+            launch_wilson_sheets(w, 0, c->cfg.Ny, st);
+            IPG_LAUNCHED(c, 4);
+            continue;
+        }
         for (int k0 = 0; k0 < c->cfg.Ny; k0 += sheets, batch++) {
             const int ns = std::min(sheets, c->cfg.Ny - k0);
             const int i = batch & 1;
@@ -1293,6 +1314,10 @@ static ipg_status init_enqueue(ipg_ctx *c, bool from_wilson) {
             IPG_CUDA(c, cudaEventRecord(c->ev_prod[i], c->stream_v));
             IPG_LAUNCHED(c, 4);
         }
+    }
+    if (side_by_side) {
+        IPG_CUDA(c, cudaEventRecord(c->ev_nuc_join, c->stream_v));
+        IPG_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_nuc_join, 0));
     }
     if (batch > 0) {
         // V_A, V_B complete before anything else on the context stream
@@ -1819,7 +1844,6 @@ ipg_status backward_inputs(ipg_ctx *c, double *grad_g2mu, double *grad_rho) {
         for (C<double> **p : {&A.b1x, &A.b2x, &A.b1y, &A.b2y, &A.vbA, &A.vbB, &A.vcur, &A.vcur2})
             IPG_TRY(dalloc(c, p, 9 * n));
         IPG_TRY(dalloc(c, &A.g2mu_bar, 2 * n));
-        IPG_TRY(dalloc(c, &A.amp2, n));
     }
     if (grad_rho && !A.rho_all) IPG_TRY(dalloc(c, &A.rho_all, 16 * (size_t)Ny * n));
     for (C<double> *p : {A.b1x, A.b2x, A.b1y, A.b2y, A.vbA, A.vbB})
@@ -1872,7 +1896,7 @@ ipg_status backward_inputs(ipg_ctx *c, double *grad_g2mu, double *grad_rho) {
         w.nucleus = (uint32_t)nuc;
         w.twiddle = c->twiddle;
         w.green = c->green;
-        w.amp = nuc ? A.amp2 : c->amp;
+        w.amp = nuc ? c->ampB : c->amp;
         w.work = work;
         w.V = vcur;
         w.no_product = 1;
