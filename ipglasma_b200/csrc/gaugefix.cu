@@ -536,13 +536,24 @@ __global__ void __launch_bounds__(GB) k_mult_bins(const double2 *planes, MultArg
     }
 }
 
-// fold the blocks' rows in block order
-__global__ void k_mult_fold(const double *partial, int blocks, double *out) {
-    for (int k = threadIdx.x; k < kMultRow; k += blockDim.x) {
-        double s = 0.;
-        for (int b = 0; b < blocks; b++) s += partial[(size_t)b * kMultRow + k];
-        out[k] = s;
+// fold the blocks' rows in block order: a thread a value, its loads sixteen
+// rows ahead of the sum (46 us with one block and one load at a time)
+constexpr int kFoldThreads = 32;
+__global__ void __launch_bounds__(kFoldThreads) k_mult_fold(const double *partial, int blocks,
+                                                            double *out) {
+    const int k = blockIdx.x * kFoldThreads + threadIdx.x;
+    if (k >= kMultRow) return;
+    double s = 0.;
+    int b = 0;
+    for (; b + 16 <= blocks; b += 16) {
+        double v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = partial[(size_t)(b + i) * kMultRow + k];
+#pragma unroll
+        for (int i = 0; i < 16; i++) s += v[i];
     }
+    for (; b < blocks; b++) s += partial[(size_t)b * kMultRow + k];
+    out[k] = s;
 }
 
 void launch_multiplicity(const State<double> &s, const MultArgs &m, double2 *planes,
@@ -553,7 +564,8 @@ void launch_multiplicity(const State<double> &s, const MultArgs &m, double2 *pla
     launch_fft2_forward(fft, 4, st);
     const int blocks = gauge_fix_blocks(m.N);
     k_mult_bins<<<blocks, GB, 0, st>>>(planes, m, partial);
-    k_mult_fold<<<1, 256, 0, st>>>(partial, blocks, out);
+    k_mult_fold<<<(kMultRow + kFoldThreads - 1) / kFoldThreads, kFoldThreads, 0, st>>>(partial, blocks,
+                                                                                     out);
 }
 
 }  // namespace ipg
