@@ -67,10 +67,16 @@ void launch_link_products(int N, C<double> *VA, C<double> *VB, C<double> *u1x,
 // by data, which would put register arrays in local memory. The row swaps
 // are applied to F as they happen, which gives the permuted right-hand side
 // that GSL forms from the permutation afterwards; F is overwritten.
-__device__ void lu_solve8(double *J, double *F, double *x, int js) {
+// The loops are unrolled, so all addresses but the pivot row's are static, and
+// the pivot row is held in registers while the rows below it are updated
+// (rolled up, every entry waited for its own shared-memory load).
+template <int js>
+__device__ __forceinline__ void lu_solve8(double *J, double *F, double *x) {
+#pragma unroll
     for (int col = 0; col < 7; col++) {
         int piv = col;
         double best = fabs(J[(col * 8 + col) * js]);
+#pragma unroll
         for (int row = col + 1; row < 8; row++) {
             double c = fabs(J[(row * 8 + col) * js]);
             if (c > best) {
@@ -79,6 +85,7 @@ __device__ void lu_solve8(double *J, double *F, double *x, int js) {
             }
         }
         if (piv != col) {
+#pragma unroll
             for (int k = 0; k < 8; k++) {
                 double t = J[(col * 8 + k) * js];
                 J[(col * 8 + k) * js] = J[(piv * 8 + k) * js];
@@ -88,26 +95,39 @@ __device__ void lu_solve8(double *J, double *F, double *x, int js) {
             F[col * js] = F[piv * js];
             F[piv * js] = t;
         }
-        const double d = J[(col * 8 + col) * js];
+        double p[8];
+#pragma unroll
+        for (int k = col; k < 8; k++) p[k] = J[(col * 8 + k) * js];
+        const double d = p[col];
         if (d != 0.0) {
+#pragma unroll
             for (int row = col + 1; row < 8; row++) {
                 const double l = J[(row * 8 + col) * js] / d;
                 J[(row * 8 + col) * js] = l;
-                for (int k = col + 1; k < 8; k++) J[(row * 8 + k) * js] -= l * J[(col * 8 + k) * js];
+#pragma unroll
+                for (int k = col + 1; k < 8; k++) J[(row * 8 + k) * js] -= l * p[k];
             }
         }
     }
+    double f[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) f[i] = F[i * js];
+#pragma unroll
     for (int i = 1; i < 8; i++) {
-        double acc = F[i * js];
-        for (int j = 0; j < i; j++) acc -= J[(i * 8 + j) * js] * F[j * js];
-        F[i * js] = acc;
+        double acc = f[i];
+#pragma unroll
+        for (int j = 0; j < i; j++) acc -= J[(i * 8 + j) * js] * f[j];
+        f[i] = acc;
     }
+#pragma unroll
     for (int i = 7; i >= 0; i--) {
-        double acc = F[i * js];
-        for (int j = i + 1; j < 8; j++) acc -= J[(i * 8 + j) * js] * F[j * js];
-        F[i * js] = acc / J[(i * 8 + i) * js];
+        double acc = f[i];
+#pragma unroll
+        for (int j = i + 1; j < 8; j++) acc -= J[(i * 8 + j) * js] * f[j];
+        f[i] = acc / J[(i * 8 + i) * js];
     }
-    for (int i = 0; i < 8; i++) x[i * js] = F[i * js];
+#pragma unroll
+    for (int i = 0; i < 8; i++) x[i * js] = f[i];
 }
 
 __device__ __forceinline__ void restart_alpha(double alpha[8], uint64_t key,
@@ -179,8 +199,8 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
     const bool mine = lid < 2 * n && !(A.redo_only && A.status[lid] != -1);
     // The iteration starts at alpha = 0, where the differenced exponentials of
     // the first Jacobian are exp(i 0.001 t^b) for every link: eight threads
-    // evaluate them for the block (nine of a link's exponentials saved; a link
-    // takes three or four iterations)
+    // evaluate them for the block (a link takes 1.5 iterations at 512^2, 3.7 at
+    // 64^2)
     double *first = newton_j + kNewtonSmem * js;
     if (!__syncthreads_or(mine)) return;
     if (threadIdx.x < 8) {
@@ -196,6 +216,13 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
     }
     __syncthreads();
     if (!mine) return;
+    // Where the last of them is the identity (the closed form gives that for
+    // exactly coinciding eigenvalues), its column of the first Jacobian is zero
+    // and the iteration takes the analytic one whatever the others are
+    bool first_good = false;
+#pragma unroll
+    for (int k = 0; k < 18; k++)
+        first_good = first_good || first[18 * 7 + k] != ((k == 0 || k == 8 || k == 16) ? 1. : 0.);
     // link order of the reference loop: per site, x then y (Init.cpp:2498-2516)
     const size_t pos = lid >> 1;
     const int dir = (int)(lid & 1);
@@ -236,8 +263,8 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
                 Fzero += fabs(f);
             }
         }
-        bool good = true;
-        for (int b = 0; b < 8; b++) {
+        bool good = total > 1 || first_good;
+        for (int b = 0; b < 8 && (total > 1 || first_good); b++) {
             const double ab = al[b * js];
             const double d = fmax(kFirstStep, fmin(10., 0.01 * fabs(ab)));
             const double ap = ab + d;
@@ -266,15 +293,17 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
         if (!good) {
             // analytic approximation (Init.cpp:3419-3431)
             const M3<double> Usold = dagger(L.U);
+#pragma unroll 1
             for (int b = 0; b < 8; b++) {
                 const M3<double> Mt = ta_mul(b, Usold);
+#pragma unroll 1
                 for (int a = 0; a < 8; a++) {
                     const M3<double> Ma = ta_mul(a, L.S);
                     J[(a * 8 + b) * js] = -2. * re_trace_mul(Ma, Mt);
                 }
             }
         }
-        lu_solve8(J, Fa, dalpha, js);
+        lu_solve8<js>(J, Fa, dalpha);
         bool ok = true;
         for (int a = 0; a < 8; a++)
             if (fabs(dalpha[a * js]) > 1e5) {
@@ -372,7 +401,7 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton_polish(NewtonArgs A) 
             im_trace_ta(Mt, tl);
             for (int a = 0; a < 8; a++) J[(a * 8 + b) * js] = -tl[a];
         }
-        lu_solve8(J, Fa, dalpha, js);
+        lu_solve8<js>(J, Fa, dalpha);
         for (int a = 0; a < 8; a++) al[a * js] -= dalpha[a * js];
     }
     // no finite residual at all: the exponent stays as the reference's
@@ -448,7 +477,7 @@ __global__ void __launch_bounds__(kFastThreads) k_newton_fast(NewtonArgs A) {
 #pragma unroll
             for (int b = 0; b < 8; b++) J[(a * 8 + b) * js] = 2. * tr[b].r;
         }
-        lu_solve8(J, Fv, dv, js);
+        lu_solve8<js>(J, Fv, dv);
         double d8[8];
         bool ok = true;
 #pragma unroll
