@@ -625,12 +625,9 @@ struct PairLoadGlobal {
 template <class Ld>
 __device__ __forceinline__ void leapfrog_pair_core(const Ld &ld, const StepCoef<float> &cf,
                                                    M3<P2> &nu, H3<float> &phin) {
-    const H3<float> phi = ld.template phi<0, 0>();
-    H3<float> pi = ld.pi();
-    H3<P2> Ed = pair_h(ld.e1(), ld.e2());
-
+    H3<float> pi;
+    H3<P2> Ed;
     if (cf.do_pe) {
-        const H3<P2> phi2 = pair_h(phi, phi);
         H3<P2> stap;
         {
             // P_do = (U_d U_o(+d)) (U_o U_d(+o))^dag: lane x of a = U_d U_o(+d)
@@ -649,7 +646,10 @@ __device__ __forceinline__ void leapfrog_pair_core(const Ld &ld, const StepCoef<
         h_traceless(stap);
         const P2 cst = P2(cf.c_e);
         const P2 cdt = P2(cf.c_pi);
+        Ed = pair_h(ld.e1(), ld.e2());
         h_axpy(Ed, cst, stap);
+        const H3<float> phi = ld.template phi<0, 0>();
+        const H3<P2> phi2 = pair_h(phi, phi);
         const H3<P2> fp = pair_h(ld.template phi<1, 0>(), ld.template phi<0, 1>());
         H3<P2> br = transport_fwd_minus<P2, true>(ld.template links<kLx, 0, 0, kLy, 0, 0>(), fp, phi2);
         h_axpy(Ed, cdt, i_commutator(br, phi2));  // i[phi~ - phi, phi] = i[phi~, phi]
@@ -658,16 +658,20 @@ __device__ __forceinline__ void leapfrog_pair_core(const Ld &ld, const StepCoef<
                                                 phi2));
         H3<float> brs = lane_h(br, 0);
         h_add(brs, lane_h(br, 1));
+        pi = ld.pi();
         h_axpy(pi, cf.c_pi, brs);
         h_traceless(Ed);
         ld.put_e(lane_h(Ed, 0), lane_h(Ed, 1));
         ld.put_pi(pi);
+    } else {
+        pi = ld.pi();
+        Ed = pair_h(ld.e1(), ld.e2());
     }
     if (cf.do_pu) {
+        phin = ld.template phi<0, 0>();
+        h_axpy(phin, cf.c_phi, pi);
         nu = taylor2_update_dev(Ed, P2(cf.c_u), ld.template links<kLx, 0, 0, kLy, 0, 0>());
         reunitarize_dev(nu);
-        phin = phi;
-        h_axpy(phin, cf.c_phi, pi);
     }
 }
 
