@@ -737,6 +737,23 @@ static_assert(SMEM <= 227 * 1024, "shared memory per block");
 }  // namespace tile
 
 
+// Programmatic dependent launch (launch_after): a step kernel may start while
+// the previous kernel of the stream is finishing; it sets up its barrier,
+// then waits here until that kernel has completed and its writes are visible.
+// Nothing before the wait touches what another kernel writes. us a step at
+// 64^2, 256^2, 512^2, 1024^2 without and with it (and the tensor maps kept by
+// the context): FP64 6.2, 18.5, 65.0, 230 -> 5.1, 17.1, 62.4, 226; FP32 10.2,
+// 16.4, 42.3, 139.6 -> 7.8, 13.1, 38.3, 131 (with leapfrog_pair_core's shorter
+// lifetimes).
+__device__ __forceinline__ void wait_previous_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// the next kernel may start its set-up once every block of this one is
+// resident or done
+__device__ __forceinline__ void allow_next_kernel() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // 32-bit shared-memory accesses by address: one value per instruction, so
 // each lands directly in its lane of a packed pair
 __device__ __forceinline__ float lds_f32(uint32_t a) {
@@ -923,24 +940,37 @@ __device__ __forceinline__ void tile32_loop(const Tiles &T, unsigned char *smem,
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + 2 * tile::STAGE);
     uint64_t *empty = full + 2;
     const int tid = threadIdx.x, r = tid >> 5, c = tid & 31;
-    const int tiles = T.total;
-    const LoadMaps *fenced = nullptr;  // thread 0: the maps acquired last
+    // Maps in global memory: lanes 0-5 of warp 0 (the issuers) each acquire and
+    // use one of the six. Maps in the kernel's parameters: thread 0 issues all
+    // loads.
+    constexpr bool kLanes = Tiles::kGlobalMaps;
+    const bool issuer = kLanes ? tid < 32 : tid == 0;
+    const CUtensorMap *fenced = nullptr;  // the map acquired last
 
     auto issue = [&](int t, int s) {
         const int e = T.find(t);
         const int N = T.n_of(e), tiles_y = N / tile::Cn, local = t - T.first_tile(e);
         const int iy0 = (local % tiles_y) * tile::Cn, ix0 = (local / tiles_y) * tile::R;
         const LoadMaps *m = T.maps_of(e);
-        if (Tiles::kGlobalMaps && m != fenced) {
-            fence_map_acquire(&m->ux);
-            fence_map_acquire(&m->uy);
-            fence_map_acquire(&m->phi);
-            fence_map_acquire(&m->e1);
-            fence_map_acquire(&m->e2);
-            fence_map_acquire(&m->pi);
-            fenced = m;
-        }
         unsigned char *st = smem + s * tile::STAGE;
+        if constexpr (kLanes) {
+            if (tid == 0) mbar_arrive_expect_tx(&full[s], tile::TX_BYTES);
+            __syncwarp();
+            if (tid < 6) {
+                const CUtensorMap *mine = &m->ux + tid;
+                if (mine != fenced) fence_map_acquire(mine);
+                fenced = mine;
+                const int to = tid == 0   ? tile::UX
+                               : tid == 1 ? tile::UY
+                               : tid == 2 ? tile::PHI
+                               : tid == 3 ? tile::E1
+                               : tid == 4 ? tile::E2
+                                          : tile::PI;
+                tma_load_3d(st + to, mine, iy0 - (tid < 2 ? 2 : (tid == 2 ? 4 : 0)),
+                            ix0 - (tid < 3 ? 1 : 0), 0, &full[s]);
+            }
+            return;
+        }
         mbar_arrive_expect_tx(&full[s], tile::TX_BYTES);
         tma_load_3d(st + tile::UX, &m->ux, iy0 - 2, ix0 - 1, 0, &full[s]);
         tma_load_3d(st + tile::UY, &m->uy, iy0 - 2, ix0 - 1, 0, &full[s]);
@@ -962,13 +992,18 @@ __device__ __forceinline__ void tile32_loop(const Tiles &T, unsigned char *smem,
             prefetch_map(&m->uy);
             prefetch_map(&m->phi);
         }
-        if (blockIdx.x < tiles) issue(blockIdx.x, 0);
-        if (blockIdx.x + gridDim.x < tiles) issue(blockIdx.x + gridDim.x, 1);
+    }
+    allow_next_kernel();
+    wait_previous_kernel();
+    const int first = blockIdx.x, end = T.total, step = gridDim.x;
+    if (issuer) {
+        if (first < end) issue(first, 0);
+        if (first + step < end) issue(first + step, 1);
     }
     __syncthreads();  // barriers initialised before anyone waits on them
 
     int i = 0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
+    for (int t = first; t < end; t += step, i++) {
         const int s = i & 1;
         const uint32_t use = (uint32_t)(i >> 1) & 1u;
         if (!mbar_wait_bounded(&full[s], use, tile::MAX_POLLS)) {
@@ -1007,12 +1042,14 @@ __device__ __forceinline__ void tile32_loop(const Tiles &T, unsigned char *smem,
             st_m3_pair(T.ux_out_of(e), T.uy_out_of(e), pos, n, nu);
             st_h(T.phi_out_of(e), pos, n, phin);
         }
-        if (tid == 0 && t + 2 * (int)gridDim.x < tiles) {
-            if (!mbar_wait_bounded(&empty[s], use, tile::MAX_POLLS)) {
+        if (issuer && t + 2 * step < end) {
+            bool released = mbar_wait_bounded(&empty[s], use, tile::MAX_POLLS);
+            if constexpr (kLanes) released = __all_sync(0xffffffffu, released);
+            if (!released) {
                 if (status) *status = 1.0;  // a warp never released the stage
                 break;
             }
-            issue(t + 2 * gridDim.x, s);
+            issue(t + 2 * step, s);
         }
     }
 }
@@ -1067,7 +1104,7 @@ __global__ void __launch_bounds__(256, 1)
 // Bound by the FP64 pipe (about 60% busy at 512^2) and the wait for the
 // stage. us a step at 64^2, 128^2, 256^2, 512^2, 1024^2: one thread a site on
 // 4 x 32 tiles 11.5, 12.3, 24.6, 77.0, 258.8; this kernel 6.2, 9.1, 18.8,
-// 65.3, 232.2. Tiles of 4 rows (two blocks an SM): 8.2, 9.0, 20.6, 67.2,
+// 65.3, 232.2 (before dependent launches). Tiles of 4 rows (two blocks an SM): 8.2, 9.0, 20.6, 67.2,
 // 230.1; of 1 row: 6.2, 10.2, 20.4, 67.8, 244.2.
 // ---------------------------------------------------------------------------
 namespace tile64 {
@@ -1085,7 +1122,8 @@ constexpr int STAGE = PI + tile::round128(9 * kS * 8);
 constexpr uint32_t TX_BYTES = 2 * 9 * kU * 16 + 9 * kP * 8 + 2 * 8 * kS * 8 + 9 * kS * 8;
 constexpr int SMEM = STAGE + 64 + 128;
 constexpr int THREADS = 2 * R * Cn;
-static_assert(3 * (SMEM + 1024) <= 228 * 1024, "three blocks per SM");
+constexpr int BLOCKS = 3;  // per SM
+static_assert(BLOCKS * (SMEM + 1024) <= 228 * 1024, "shared memory of the SM");
 }  // namespace tile64
 
 // Explicit shared-memory loads by 32-bit address, so that a link used twice
@@ -1237,41 +1275,61 @@ __device__ __forceinline__ void leapfrog_role64(uint32_t st, int r, int c, int d
     }
 }
 
-// One 2 x 32 tile of the FP64 step: load the stage, wait, clamp the halo on
-// edge tiles, advance the tile's sites. tx, ty: the tile in the event's
-// N/2 x N/32 grid.
-template <bool GLOBAL_MAPS>
-__device__ __forceinline__ void tile64_body(const LoadMaps *maps, int N, int tx, int ty,
-                                            const StepCoef<double> &cf, double *status,
-                                            const State<double> &s, C<double> *ux_out,
-                                            C<double> *uy_out, double *phi_out) {
+// Load k (0 .. 5: Ux, Uy, phi, E1, E2, pi) of the stage at tile (ix0, iy0).
+// Links are pairs of 8-byte words: column iy0-1 is word 2 (iy0 - 1).
+__device__ __forceinline__ void load_box64(unsigned char *smem, const CUtensorMap *map, int k,
+                                           int ix0, int iy0, uint64_t *full) {
+    const int to = k == 0   ? tile64::UX
+                   : k == 1 ? tile64::UY
+                   : k == 2 ? tile64::PHI
+                   : k == 3 ? tile64::E1
+                   : k == 4 ? tile64::E2
+                            : tile64::PI;
+    tma_load_3d(smem + to, map, k < 2 ? 2 * (iy0 - 1) : (k == 2 ? iy0 - 2 : iy0),
+                k < 3 ? ix0 - 1 : ix0, 0, full);
+}
+
+// A thread's share of the staged tile: a warp is 16 sites of one row, lanes
+// 0-15 direction x, lanes 16-31 direction y.
+__device__ __forceinline__ void compute_stage64(const unsigned char *smem, int ix0, int iy0,
+                                                const StepCoef<double> &cf,
+                                                const State<double> &s, C<double> *ux_out,
+                                                C<double> *uy_out, double *phi_out, int N) {
+    const int tid = threadIdx.x, w = tid >> 5, dir = (tid >> 4) & 1;
+    const int r = w >> 1, c = (w & 1) * 16 + (tid & 15);
+    leapfrog_role64(smem_addr(smem), r, c, dir, cf, s, dir ? uy_out : ux_out, phi_out, N,
+                    ix0 + r, iy0 + c);
+}
+
+// One block per tile of the event's N/2 x N/32 grid.
+// (THREADS, 3): what shared memory allows, 168 registers a thread
+__global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
+    k_leapfrog_tile64(const __grid_constant__ LoadMaps maps, int N, StepCoef<double> cf,
+                      double *status, State<double> s, C<double> *ux_out, C<double> *uy_out,
+                      double *phi_out) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint32_t pad = (128u - (smem_addr(smem_raw) & 127u)) & 127u;
     unsigned char *smem = smem_raw + pad;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + tile64::STAGE);
     int *abort_flag = reinterpret_cast<int *>(full + 1);
-    const int iy0 = ty * tile64::Cn, ix0 = tx * tile64::R;
+    const int tiles_y = N / tile64::Cn;
+    const int iy0 = (blockIdx.x % tiles_y) * tile64::Cn, ix0 = (blockIdx.x / tiles_y) * tile64::R;
     const int tid = threadIdx.x;
     if (tid == 0) {
         mbar_init(full, 1);
         *abort_flag = 0;
         fence_barrier_init();
-        if (GLOBAL_MAPS) {
-            fence_map_acquire(&maps->ux);
-            fence_map_acquire(&maps->uy);
-            fence_map_acquire(&maps->phi);
-            fence_map_acquire(&maps->e1);
-            fence_map_acquire(&maps->e2);
-            fence_map_acquire(&maps->pi);
-        }
+    }
+    allow_next_kernel();
+    wait_previous_kernel();
+    if (tid == 0) {
         mbar_arrive_expect_tx(full, tile64::TX_BYTES);
-        // links as pairs of 8-byte words: column iy0-1 is word 2 (iy0 - 1)
-        tma_load_3d(smem + tile64::UX, &maps->ux, 2 * (iy0 - 1), ix0 - 1, 0, full);
-        tma_load_3d(smem + tile64::UY, &maps->uy, 2 * (iy0 - 1), ix0 - 1, 0, full);
-        tma_load_3d(smem + tile64::PHI, &maps->phi, iy0 - 2, ix0 - 1, 0, full);
-        tma_load_3d(smem + tile64::E1, &maps->e1, iy0, ix0, 0, full);
-        tma_load_3d(smem + tile64::E2, &maps->e2, iy0, ix0, 0, full);
-        tma_load_3d(smem + tile64::PI, &maps->pi, iy0, ix0, 0, full);
+        load_box64(smem, &maps.ux, 0, ix0, iy0, full);
+        load_box64(smem, &maps.uy, 1, ix0, iy0, full);
+        load_box64(smem, &maps.phi, 2, ix0, iy0, full);
+        load_box64(smem, &maps.e1, 3, ix0, iy0, full);
+        load_box64(smem, &maps.e2, 4, ix0, iy0, full);
+        load_box64(smem, &maps.pi, 5, ix0, iy0, full);
     }
     __syncthreads();
     if (!mbar_wait_bounded(full, 0, tile::MAX_POLLS)) *abort_flag = 1;
@@ -1280,42 +1338,73 @@ __device__ __forceinline__ void tile64_body(const LoadMaps *maps, int N, int tx,
         if (tid == 0 && status) *status = 1.0;
         return;
     }
-    // a warp is 16 sites of one row: lanes 0-15 direction x, 16-31 direction y
-    const int w = tid >> 5, dir = (tid >> 4) & 1;
-    const int r = w >> 1, c = (w & 1) * 16 + (tid & 15);
-    leapfrog_role64(smem_addr(smem), r, c, dir, cf, s, dir ? uy_out : ux_out, phi_out, N,
-                        ix0 + r, iy0 + c);
+    compute_stage64(smem, ix0, iy0, cf, s, ux_out, uy_out, phi_out, N);
 }
 
-// (THREADS, 3): what shared memory allows, 168 registers a thread
-__global__ void __launch_bounds__(tile64::THREADS, 3)
-    k_leapfrog_tile64(const __grid_constant__ LoadMaps maps, int N, StepCoef<double> cf,
-                      double *status, State<double> s, C<double> *ux_out, C<double> *uy_out,
-                      double *phi_out) {
-    const int tiles_y = N / tile64::Cn;
-    tile64_body<false>(&maps, N, blockIdx.x / tiles_y, blockIdx.x % tiles_y, cf, status, s,
-                       ux_out, uy_out, phi_out);
-}
-
-// The FP64 batch over the TMA tiles: one block per tile of the concatenated
-// tile lists; the block reads its event's descriptor and tensor maps from
-// global memory.
-__global__ void __launch_bounds__(tile64::THREADS, 3)
+// The FP64 batch over the TMA tiles: BLOCKS persistent blocks an SM, each with
+// consecutive tiles of the concatenated tile lists, so that it meets few events:
+// a new event costs the acquire of its tensor maps in global memory. The step's
+// descriptors and the tile prefix sums are copied to shared memory behind the
+// stage, since a thread reads its coefficients in the middle of the update.
+// ms for 52 steps of 3 x 512^2 + 8 x 128^2, 4 x 512^2 + 2 x 128^2 and
+// 4 x 256^2 + 10 x 64^2: one block per tile with its own acquires and
+// descriptor reads 21.5, 25.3, 7.3; persistent blocks on every gridDim.x-th
+// tile 15.6, 17.5, 6.1; consecutive tiles 14.9, 17.4, 5.4; descriptors in
+// shared memory as well 13.5, 15.7, 4.8.
+__global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
     k_leapfrog_tile64_batch(const BatchEvent<double> *__restrict__ evs, int n_events,
-                            const int *__restrict__ tile_begin, const LoadMaps *__restrict__ maps,
-                            double *status) {
-    const int t = blockIdx.x;
-    int lo = 0, hi = n_events - 1;  // last e with tile_begin[e] <= t
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(tile_begin + mid) <= t) lo = mid;
-        else hi = mid - 1;
+                            const int *__restrict__ tile_begin, int total_tiles,
+                            const LoadMaps *__restrict__ maps, double *status) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const uint32_t pad = (128u - (smem_addr(smem_raw) & 127u)) & 127u;
+    unsigned char *smem = smem_raw + pad;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + tile64::STAGE);
+    BatchEvent<double> *s_ev =
+        reinterpret_cast<BatchEvent<double> *>(smem + tile64::STAGE + 64);
+    int *s_begin = reinterpret_cast<int *>(s_ev + n_events);
+    {
+        const int words = n_events * (int)(sizeof(BatchEvent<double>) / sizeof(int));
+        const int *src = reinterpret_cast<const int *>(evs);
+        int *dst = reinterpret_cast<int *>(s_ev);
+        for (int w = threadIdx.x; w < words; w += tile64::THREADS) dst[w] = src[w];
     }
-    const BatchEvent<double> &E = evs[lo];
-    if (!E.active) return;
-    const int N = E.N, tiles_y = N / tile64::Cn, local = t - __ldg(tile_begin + lo);
-    tile64_body<true>(maps + 2 * lo + E.map_sel, N, local / tiles_y, local % tiles_y, E.cf,
-                      status, E.s, E.ux_out, E.uy_out, E.phi_out);
+    for (int e = threadIdx.x; e <= n_events; e += tile64::THREADS) s_begin[e] = tile_begin[e];
+    if (threadIdx.x == 0) {
+        mbar_init(full, 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    allow_next_kernel();
+    wait_previous_kernel();
+    uint32_t phase = 0;
+    int e = 0, fenced = -1;
+    const int end = (int)((long long)total_tiles * (blockIdx.x + 1) / gridDim.x);
+    for (int t = (int)((long long)total_tiles * blockIdx.x / gridDim.x); t < end; t++) {
+        while (s_begin[e + 1] <= t) e++;
+        const BatchEvent<double> &E = s_ev[e];
+        if (!E.active) continue;
+        const int N = E.N, tiles_y = N / tile64::Cn, local = t - s_begin[e];
+        const int iy0 = (local % tiles_y) * tile64::Cn, ix0 = (local / tiles_y) * tile64::R;
+        const int tid = threadIdx.x;
+        if (tid < 32) {
+            if (tid == 0) mbar_arrive_expect_tx(full, tile64::TX_BYTES);
+            __syncwarp();
+            if (tid < 6) {
+                const CUtensorMap *mine = &maps[2 * e + E.map_sel].ux + tid;
+                if (fenced != e) fence_map_acquire(mine);
+                fenced = e;
+                load_box64(smem, mine, tid, ix0, iy0, full);
+            }
+        }
+        const bool arrived = mbar_wait_bounded(full, phase, tile::MAX_POLLS);
+        phase ^= 1;
+        if (arrived)
+            compute_stage64(smem, ix0, iy0, E.cf, E.s, E.ux_out, E.uy_out, E.phi_out, N);
+        if (__syncthreads_or(!arrived)) {  // else the stage is free
+            if (threadIdx.x == 0 && status) *status = 1.0;
+            return;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1369,9 +1458,32 @@ __global__ void __launch_bounds__(32 * TX, 8 / TX)
     }
 }
 
+// Launch with programmatic stream serialisation: the kernel calls
+// wait_previous_kernel itself.
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                  cudaStream_t st, A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 template <typename T>
 size_t batch_smem(int n_events) {
     return sizeof(BatchEvent<T>) * n_events + sizeof(int) * (n_events + 1);
+}
+
+// shared memory of the FP64 tile batch kernel, in the same way: one stage
+size_t tile64_batch_smem(int n_events) {
+    return (size_t)tile64::SMEM + batch_smem<double>(n_events);
 }
 
 // shared memory of the FP32 TMA batch kernel: two stages, the barriers, the
@@ -1408,12 +1520,13 @@ int batch_max_blocks_per_sm(int variant, int n_events) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile_batch, 256, smem);
             return nb > 1 ? 1 : nb;  // persistent: one block per SM
         } else {
+            const size_t smem = tile64_batch_smem(n_events);
+            if (smem > 227 * 1024) return 0;  // too many events for the descriptors
             cudaFuncSetAttribute(k_leapfrog_tile64_batch,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, tile64::SMEM);
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile64_batch,
-                                                          tile64::THREADS,
-                                                          tile64::SMEM);
-            return nb > 0 ? 1 : 0;  // one block per tile: the grid is the tile count
+                                                          tile64::THREADS, smem);
+            return nb > 0 ? 1 : 0;  // launched with BLOCKS blocks an SM
         }
     }
     const int threads = 32 * batch_tile_rows<T>(variant);
@@ -1430,11 +1543,13 @@ void launch_leapfrog_batch(const BatchEvent<T> *d_evs, int n_events, const int *
         if constexpr (sizeof(T) == 4) {
             const size_t smem = tile_batch_smem(n_events);
             // imag = 4: the byte offset of a link's imaginary part
-            k_leapfrog_tile_batch<<<grid < total_tiles ? grid : total_tiles, 256, smem, st>>>(
-                d_evs, n_events, d_tile_begin, total_tiles, d_maps, status, 4u);
+            launch_after(k_leapfrog_tile_batch, grid < total_tiles ? grid : total_tiles, 256, smem,
+                         st, d_evs, n_events, d_tile_begin, total_tiles, d_maps, status, 4u);
         } else {
-            k_leapfrog_tile64_batch<<<total_tiles, tile64::THREADS, tile64::SMEM, st>>>(
-                d_evs, n_events, d_tile_begin, d_maps, status);
+            const int blocks = tile64::BLOCKS * grid;
+            launch_after(k_leapfrog_tile64_batch, blocks < total_tiles ? blocks : total_tiles,
+                         tile64::THREADS, tile64_batch_smem(n_events), st, d_evs, n_events, d_tile_begin,
+                         total_tiles, d_maps, status);
         }
         return;
     }
@@ -1542,18 +1657,20 @@ bool use_tile_kernel() {
 // false if a tensor map could not be encoded (nothing launched)
 bool launch_leapfrog_tile(int N, const State<float> &s, C<float> *ux_out, C<float> *uy_out,
                           float *phi_out, const StepCoef<float> &cf, double *status,
-                          cudaStream_t st) {
+                          cudaStream_t st, const LoadMaps *maps) {
     using namespace tile;
     LoadMaps m;
-    if (!encode_step_maps<float>(N, s, &m)) return false;
+    if (maps)
+        m = *maps;
+    else if (!encode_step_maps<float>(N, s, &m))
+        return false;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_leapfrog_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     const int tiles = (N / R) * (N / Cn);
     // imag = 4: the byte offset of a link's imaginary part
-    k_leapfrog_tile<<<tiles < sms ? tiles : sms, 256, SMEM, st>>>(m, N, cf, status, 4u, s, ux_out,
-                                                                  uy_out, phi_out);
+    launch_after(k_leapfrog_tile, tiles < sms ? tiles : sms, 256, SMEM, st, m, N, cf, status, 4u, s,
+                 ux_out, uy_out, phi_out);
     return true;
 }
 
@@ -1573,22 +1690,33 @@ bool use_tile64_kernel() {
 bool launch_leapfrog_tile64(int N, const State<double> &links, const State<double> &ein,
                             const State<double> &out, C<double> *ux_out, C<double> *uy_out,
                             double *phi_out, const StepCoef<double> &cf, double *status,
-                            cudaStream_t st) {
+                            cudaStream_t st, const LoadMaps *maps = nullptr) {
     using namespace tile64;
     LoadMaps m;
-    if (!encode_maps64(N, links, ein, &m)) return false;
-    cudaFuncSetAttribute(k_leapfrog_tile64, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    k_leapfrog_tile64<<<(N / R) * (N / Cn), THREADS, SMEM, st>>>(m, N, cf, status, out, ux_out,
-                                                                 uy_out, phi_out);
+    if (maps)
+        m = *maps;
+    else if (!encode_maps64(N, links, ein, &m))
+        return false;
+    launch_after(k_leapfrog_tile64, (N / R) * (N / Cn), THREADS, SMEM, st, m, N, cf, status, out,
+                 ux_out, uy_out, phi_out);
     return true;
 }
 
 }  // namespace
 
+cudaError_t prepare_leapfrog() {
+    cudaError_t e = cudaFuncSetAttribute(
+        k_leapfrog_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, tile::SMEM);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_leapfrog_tile64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                tile64::SMEM);
+}
+
 template <typename T>
 void launch_leapfrog(const EventGeom *d_ev, int N, const State<T> &s,
                      C<T> *ux_out, C<T> *uy_out, T *phi_out,
-                     const StepCoef<T> &cf, bool reunit, cudaStream_t st, double *status) {
+                     const StepCoef<T> &cf, bool reunit, cudaStream_t st, double *status,
+                     const LoadMaps *maps) {
     // FP64 runs two threads per site from shared-memory tiles filled by TMA
     // (k_leapfrog_tile64), or one thread per site from plain loads. FP32 runs both directions of a site in the
     // two lanes of packed FP32 instructions, from shared-memory tiles filled
@@ -1598,7 +1726,7 @@ void launch_leapfrog(const EventGeom *d_ev, int N, const State<T> &s,
             // N is a power of two >= 32: the tiles cover the lattice exactly
             (void)reunit;
             if (use_tile_kernel() &&
-                launch_leapfrog_tile(N, s, ux_out, uy_out, phi_out, cf, status, st))
+                launch_leapfrog_tile(N, s, ux_out, uy_out, phi_out, cf, status, st, maps))
                 return;
             k_leapfrog_pair<<<dim3(N / 32, N / 8), 256, 0, st>>>(d_ev, s, ux_out, uy_out, phi_out,
                                                                  cf);
@@ -1607,7 +1735,7 @@ void launch_leapfrog(const EventGeom *d_ev, int N, const State<T> &s,
     }
     if constexpr (sizeof(T) == 8) {
         if (N >= 32 && !reunit && use_tile64_kernel() &&
-            launch_leapfrog_tile64(N, s, s, s, ux_out, uy_out, phi_out, cf, status, st))
+            launch_leapfrog_tile64(N, s, s, s, ux_out, uy_out, phi_out, cf, status, st, maps))
             return;
     }
     launch_leapfrog_site(d_ev, N, s, ux_out, uy_out, phi_out, cf, reunit, st);
@@ -1688,9 +1816,10 @@ template void launch_inverse_se<double>(int, const State<double> &, const State<
 
 template void launch_leapfrog<double>(const EventGeom *, int, const State<double> &,
                                       C<double> *, C<double> *, double *,
-                                      const StepCoef<double> &, bool, cudaStream_t, double *);
+                                      const StepCoef<double> &, bool, cudaStream_t, double *,
+                                      const LoadMaps *);
 template void launch_leapfrog<float>(const EventGeom *, int, const State<float> &, C<float> *,
                                      C<float> *, float *, const StepCoef<float> &, bool,
-                                     cudaStream_t, double *);
+                                     cudaStream_t, double *, const LoadMaps *);
 
 }  // namespace ipg

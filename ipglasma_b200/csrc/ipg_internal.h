@@ -44,13 +44,19 @@ inline void set_derived(StepCoef<T> &cf) {
     cf.c_phi = (cf.tau + cf.dt_pu / T(2)) * cf.dt_pu;
 }
 
-// status (may be null): set to 1 if a wait of the FP32 tile kernel hit its
-// limit (the step is then incomplete)
+struct LoadMaps;
+// Once per device before the first leapfrog launch there (ipg_create): the
+// tile kernels' shared-memory limits.
+cudaError_t prepare_leapfrog();
+// status (may be null): set to 1 if a wait of the tile kernel hit its limit
+// (the step is then incomplete). maps (may be null): the tensor maps of s, as
+// encode_step_maps makes them; encoding six maps takes about as long as a
+// launch, so a caller that steps the same buffers again and again keeps them.
 template <typename T>
 void launch_leapfrog(const EventGeom *d_ev, int N, const State<T> &s,
                      C<T> *ux_out, C<T> *uy_out, T *phi_out,
                      const StepCoef<T> &cf, bool reunit, cudaStream_t st,
-                     double *status = nullptr);
+                     double *status = nullptr, const LoadMaps *maps = nullptr);
 
 // One FP64 step from the state `in` into the separate state `out` (all six
 // fields written; `in` is left unchanged)
