@@ -35,6 +35,7 @@ struct ipg_ctx {
     int itmax = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t evo0 = nullptr, evo1 = nullptr;  // around the evolution of a run
     // Wilson-line stage: the exponential products of a sheet batch run on
     // stream_v while the next batch's Poisson transforms run on stream, into
     // the other of two work buffers (work, work2)
@@ -435,7 +436,7 @@ ipg_status step32_into(ipg_ctx *c, const State<float> &in, const State<float> &o
     return IPG_OK;
 }
 
-// coefficients of launch s of run_evolution (0: tau = 0 half step)
+// coefficients of launch s of evolution_enqueue (0: tau = 0 half step)
 StepCoef<double> evolution_coef(const ipg_ctx *c, int s) {
     StepCoef<double> cf;
     cf.tau = s * c->dtau;
@@ -482,20 +483,29 @@ bool in_ecc_window(int N, int i, int j) { return i >= 2 && i < N - 2 && j >= 2 &
 // The leapfrog schedule of Evolution::run up to it = itmax - 1: the tau = 0
 // half step of phi and U (Evolution.cpp:393-394), then full steps
 // it = 1 .. itmax-1 (416-421).
-ipg_status run_evolution(ipg_ctx *c) {
+// All steps of a run, enqueued on the context's stream; evolution_finish waits
+// for the stream and takes the time. ipg_run enqueues the observables in
+// between, so that the GPU does not wait for the host after the last step.
+ipg_status evolution_enqueue(ipg_ctx *c) {
     const int itmax = c->itmax;
     const double dtau = c->dtau;
-    IPG_CUDA(c, cudaEventRecord(c->ev0, c->stream));
+    IPG_CUDA(c, cudaEventRecord(c->evo0, c->stream));
     IPG_TRY(step(c, 0., dtau, dtau, 0, 1));
     c->half_done = true;
     for (int it = 1; it < itmax; it++) {
         IPG_TRY(step(c, it * dtau, dtau, dtau, 1, 1));
         c->it = it;
     }
-    IPG_CUDA(c, cudaEventRecord(c->ev1, c->stream));
+    IPG_CUDA(c, cudaEventRecord(c->evo1, c->stream));
+    return IPG_OK;
+}
+
+ipg_status evolution_finish(ipg_ctx *c) {
     IPG_TRY(sync(c));
-    c->last_leapfrog_ms = elapsed(c);
-    c->last_leapfrog_launches = itmax;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, c->evo0, c->evo1);
+    c->last_leapfrog_ms = ms;
+    c->last_leapfrog_launches = c->itmax;
     return IPG_OK;
 }
 
@@ -812,6 +822,8 @@ ipg_status ipg_create(const ipg_config *cfg, ipg_ctx **out) {
         IPG_CUDA(c, cudaEventCreateWithFlags(&c->ev_prod[i], cudaEventDisableTiming));
     }
     IPG_CUDA(c, cudaEventCreate(&c->ev0));
+    IPG_CUDA(c, cudaEventCreate(&c->evo0));
+    IPG_CUDA(c, cudaEventCreate(&c->evo1));
     IPG_CUDA(c, cudaEventCreate(&c->ev1));
     for (cudaEvent_t &x : c->ie) IPG_CUDA(c, cudaEventCreate(&x));
 
@@ -941,6 +953,8 @@ ipg_status ipg_destroy(ipg_ctx *ctx) {
     for (cudaEvent_t x : ctx->ie)
         if (x) cudaEventDestroy(x);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
+    if (ctx->evo0) cudaEventDestroy(ctx->evo0);
+    if (ctx->evo1) cudaEventDestroy(ctx->evo1);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->stream_copy) {
         cudaStreamSynchronize(ctx->stream_copy);
@@ -1468,8 +1482,9 @@ ipg_status ipg_run(ipg_ctx *c, ipg_result *res) {
     if (!c) return IPG_ERR_BAD_CONFIG;
     if (!c->initialized || c->half_done || c->finished)
         return fail(c, IPG_ERR_STATE, "ipg_run needs fresh initial fields");
-    IPG_TRY(run_evolution(c));
+    IPG_TRY(evolution_enqueue(c));
     IPG_TRY(observables_enqueue(c));
+    IPG_TRY(evolution_finish(c));
     return observables_finish(c, res);
 }
 
@@ -1536,7 +1551,8 @@ ipg_status ipg_run_multiplicity(ipg_ctx *c, const ipg_multiplicity_params *p, ip
         IPG_TRY(ipg_evolve(c, itmax - 2));
         ms += c->last_leapfrog_ms;
     } else {
-        IPG_TRY(run_evolution(c));
+        IPG_TRY(evolution_enqueue(c));
+        IPG_TRY(evolution_finish(c));
         ms += c->last_leapfrog_ms;
     }
     c->last_leapfrog_ms = ms;
@@ -2410,7 +2426,7 @@ ipg_status upload_tiles(ipg_batch *b, int variant) {
 }
 
 // descriptors of steps [0, steps) for every event, following the schedule of
-// run_evolution: step 0 is the tau = 0 half step of phi and U, step k > 0 the
+// evolution_enqueue: step 0 is the tau = 0 half step of phi and U, step k > 0 the
 // full step it = k. U/phi buffers alternate after every step. With
 // full_first, step 0 is laid out on the current buffers but carries the
 // coefficients of the full step it = 1 (the step the tuner times: it reads
