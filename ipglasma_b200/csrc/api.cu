@@ -539,8 +539,8 @@ ipg_status observables_enqueue(ipg_ctx *c) {
     // FP32 contexts: T^munu reads the FP32 state directly
     ta.from32 = is_fp32(c) ? 1 : 0;
     ta.s32 = c->s32;
-    launch_tmunu(ta, c->stream);
-    IPG_LAUNCHED(c, 7);
+    const int parts = launch_tmunu(ta, c->stream);
+    IPG_LAUNCHED(c, parts);
     LandauArgs la;
     la.N = N;
     la.tau_fm = itmax * dtau * c->a;

@@ -302,7 +302,8 @@ struct TmunuArgs {
     State<float> s32{};
     int from32 = 0;
 };
-void launch_tmunu(const TmunuArgs &a, cudaStream_t st);
+// returns the launches it made
+int launch_tmunu(const TmunuArgs &a, cudaStream_t st);
 // T^tautau, T^xx, T^yy, T^etaeta only
 void launch_tmunu_diag(const TmunuArgs &a, cudaStream_t st);
 

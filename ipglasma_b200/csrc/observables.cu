@@ -83,7 +83,7 @@ __device__ __forceinline__ M3<double> tr_bwd(const M3<double> &u,
 
 // diagonal components: T^tautau, T^xx, T^yy, T^etaeta (Evolution.cpp:735-899)
 template <typename S>
-__global__ void k_tmunu_diag(TmunuArgs A) {
+__device__ __forceinline__ void tmunu_diag(const TmunuArgs &A) {
     const int N = A.N;
     const size_t n = (size_t)N * N;
     const size_t pos = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -183,7 +183,7 @@ __device__ __forceinline__ OffdiagGeom offdiag_geom(int N, size_t pos) {
 }
 
 template <int PART, typename S>
-__global__ void __launch_bounds__(128) k_tmunu_offdiag(TmunuArgs A) {
+__device__ __forceinline__ void tmunu_offdiag(const TmunuArgs &A) {
     const int N = A.N;
     const size_t n = (size_t)N * N;
     const size_t pos = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -346,6 +346,11 @@ __global__ void __launch_bounds__(128) k_tmunu_offdiag(TmunuArgs A) {
     }
 }
 
+template <typename S>
+__global__ void k_tmunu_diag(const __grid_constant__ TmunuArgs A) {
+    tmunu_diag<S>(A);
+}
+
 void launch_tmunu_diag(const TmunuArgs &a, cudaStream_t st) {
     const size_t n = (size_t)a.N * a.N;
     if (a.from32)
@@ -354,10 +359,46 @@ void launch_tmunu_diag(const TmunuArgs &a, cudaStream_t st) {
         k_tmunu_diag<double><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(a);
 }
 
+template <int PART, typename S>
+__global__ void __launch_bounds__(128) k_tmunu_offdiag(const __grid_constant__ TmunuArgs A) {
+    tmunu_offdiag<PART, S>(A);
+}
+
+// Small lattices: the parts that read the fields only in one launch, then the
+// two that finish the sums of parts 0 and 2 in another; blockIdx.y is the part.
+// A part alone has 32 blocks at 64^2, and seven launches one after the other
+// leave most of the GPU idle.
+template <typename S, int PHASE>
+__global__ void __launch_bounds__(128) k_tmunu(const __grid_constant__ TmunuArgs A) {
+    if constexpr (PHASE == 0) {
+        switch (blockIdx.y) {
+            case 0: tmunu_offdiag<0, S>(A); break;
+            case 1: tmunu_offdiag<2, S>(A); break;
+            case 2: tmunu_diag<S>(A); break;
+            case 3: tmunu_offdiag<4, S>(A); break;
+            default: tmunu_offdiag<5, S>(A); break;
+        }
+    } else {
+        if (blockIdx.y == 0)
+            tmunu_offdiag<1, S>(A);
+        else
+            tmunu_offdiag<3, S>(A);
+    }
+}
+
 template <typename S>
-static void launch_tmunu_t(const TmunuArgs &a, cudaStream_t st) {
+static int launch_tmunu_t(const TmunuArgs &a, cudaStream_t st) {
     const size_t n = (size_t)a.N * a.N;
     const unsigned b = (unsigned)((n + 127) / 128);
+    // side by side while one part does not give every SM a block: us for all
+    // observables one after the other and side by side, 64^2 178 and 149, 128^2
+    // 197 and 197; above that the mixed parts spill more and share the L1 worse:
+    // 256^2 295 and 309, 512^2 FP32 854 and 872
+    if (b <= 148) {
+        k_tmunu<S, 0><<<dim3(b, 5), 128, 0, st>>>(a);
+        k_tmunu<S, 1><<<dim3(b, 2), 128, 0, st>>>(a);
+        return 2;
+    }
     k_tmunu_diag<S><<<b, 128, 0, st>>>(a);
     k_tmunu_offdiag<0, S><<<b, 128, 0, st>>>(a);
     k_tmunu_offdiag<1, S><<<b, 128, 0, st>>>(a);
@@ -365,13 +406,11 @@ static void launch_tmunu_t(const TmunuArgs &a, cudaStream_t st) {
     k_tmunu_offdiag<3, S><<<b, 128, 0, st>>>(a);
     k_tmunu_offdiag<4, S><<<b, 128, 0, st>>>(a);
     k_tmunu_offdiag<5, S><<<b, 128, 0, st>>>(a);
+    return 7;
 }
 
-void launch_tmunu(const TmunuArgs &a, cudaStream_t st) {
-    if (a.from32)
-        launch_tmunu_t<float>(a, st);
-    else
-        launch_tmunu_t<double>(a, st);
+int launch_tmunu(const TmunuArgs &a, cudaStream_t st) {
+    return a.from32 ? launch_tmunu_t<float>(a, st) : launch_tmunu_t<double>(a, st);
 }
 
 }  // namespace ipg
