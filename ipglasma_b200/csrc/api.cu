@@ -2408,6 +2408,13 @@ int tma_variant(const ipg_batch *b) {
     return b->fp32 ? batch_plain_variants<float>() : batch_plain_variants<double>();
 }
 
+// whether (variant, blocks per SM) can run this batch
+bool shape_fits(const ipg_batch *b, const std::pair<int, int> &shape) {
+    const int v = shape.first;
+    if (v < 0 || v >= n_variants(b) || (v == tma_variant(b) && !b->d_maps)) return false;
+    return shape.second >= 1 && shape.second <= max_blocks(b, v);
+}
+
 ipg_status upload_tiles(ipg_batch *b, int variant) {
     if (b->tiles_variant == variant) return IPG_OK;
     const int E = (int)b->ev.size();
@@ -2620,7 +2627,8 @@ ipg_status ipg_batch_create(ipg_ctx *const *events, int count, ipg_batch **out) 
         IPG_BCUDA(b, cudaStreamSynchronize(b->stream));
     }
     const auto it = tune_cache().find(tune_key(b));
-    if (it != tune_cache().end()) {
+    // (a shape saved by another build may not fit this one's kernels)
+    if (it != tune_cache().end() && shape_fits(b, it->second)) {
         b->variant = it->second.first;
         b->blocks_per_sm = it->second.second;
         b->tuned = true;
@@ -2695,7 +2703,7 @@ ipg_status ipg_batch_tune(ipg_batch *b, ipg_tune_report *rep) {
         rep->from_cache = from_cache;
     };
     auto hit = tune_cache().find(key);
-    if (hit != tune_cache().end()) {
+    if (hit != tune_cache().end() && shape_fits(b, hit->second)) {
         b->variant = hit->second.first;
         b->blocks_per_sm = hit->second.second;
         b->grid = b->blocks_per_sm * b->sms;

@@ -19,6 +19,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 
 #include "fields.cuh"
 #include "ipg_internal.h"
@@ -733,7 +734,8 @@ constexpr uint32_t TX_BYTES = 2 * 9 * kU * 8 + 9 * kP * 4 + 2 * 8 * kS * 4 + 9 *
 constexpr int SMEM = 2 * STAGE + 64 + 128;  // two stages, four barriers, alignment slack
 constexpr uint32_t MAX_POLLS = 1u << 22;
 static_assert(STAGE % 128 == 0, "stage alignment");
-static_assert(SMEM <= 227 * 1024, "shared memory per block");
+constexpr int SMEM_LIMIT = 227 * 1024;  // per block
+static_assert(SMEM <= SMEM_LIMIT, "shared memory per block");
 }  // namespace tile
 
 
@@ -1514,16 +1516,12 @@ int batch_max_blocks_per_sm(int variant, int n_events) {
     if (variant == batch_plain_variants<T>()) {
         if constexpr (sizeof(T) == 4) {
             const size_t smem = tile_batch_smem(n_events);
-            if (smem > 227 * 1024) return 0;  // too many events for the descriptors
-            cudaFuncSetAttribute(k_leapfrog_tile_batch,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem > tile::SMEM_LIMIT) return 0;  // too many events for the descriptors
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile_batch, 256, smem);
             return nb > 1 ? 1 : nb;  // persistent: one block per SM
         } else {
             const size_t smem = tile64_batch_smem(n_events);
-            if (smem > 227 * 1024) return 0;  // too many events for the descriptors
-            cudaFuncSetAttribute(k_leapfrog_tile64_batch,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem > tile::SMEM_LIMIT) return 0;  // too many events for the descriptors
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile64_batch,
                                                           tile64::THREADS, smem);
             return nb > 0 ? 1 : 0;  // launched with BLOCKS blocks an SM
@@ -1705,11 +1703,19 @@ bool launch_leapfrog_tile64(int N, const State<double> &links, const State<doubl
 }  // namespace
 
 cudaError_t prepare_leapfrog() {
-    cudaError_t e = cudaFuncSetAttribute(
-        k_leapfrog_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, tile::SMEM);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_leapfrog_tile64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                tile64::SMEM);
+    // the batch kernels: the limit itself, since batches of several sizes may
+    // be alive at once
+    const std::pair<const void *, int> kernels[] = {
+        {(const void *)k_leapfrog_tile, tile::SMEM},
+        {(const void *)k_leapfrog_tile64, tile64::SMEM},
+        {(const void *)k_leapfrog_tile_batch, tile::SMEM_LIMIT},
+        {(const void *)k_leapfrog_tile64_batch, tile::SMEM_LIMIT}};
+    for (auto &k : kernels) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, k.second);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 template <typename T>

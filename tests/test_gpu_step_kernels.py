@@ -82,3 +82,20 @@ def test_batch_matches_single_events(sizes, prec):
                 assert np.array_equal(ev.get_field(getattr(ipg, f)), x), (ev.N, f)
     for ev in events:
         ev.close()
+
+
+@pytest.mark.parametrize("prec", [ipg.FP64, ipg.FP32])
+def test_a_smaller_batch_beside_a_larger_one(prec):
+    """The larger batch needs more shared memory a block; making the smaller
+    one must not lower the limit of the kernel that both use."""
+    large = [make(prec, 32, 40 + k) for k in range(12)]
+    small = [make(prec, 32, 60)]
+    with ipg.Batch(large) as b, ipg.Batch(small) as c:
+        first = b.run()
+        second = c.run()
+    ev = make(prec, 32, 40)
+    assert ev.run().E_T == first[0].E_T
+    ev.close()
+    assert np.isfinite(second[0].E_T)
+    for ev in large + small:
+        ev.close()
