@@ -734,6 +734,7 @@ constexpr uint32_t TX_BYTES = 2 * 9 * kU * 8 + 9 * kP * 4 + 2 * 8 * kS * 4 + 9 *
 constexpr int SMEM = 2 * STAGE + 64 + 128;  // two stages, four barriers, alignment slack
 constexpr uint32_t MAX_POLLS = 1u << 22;
 static_assert(STAGE % 128 == 0, "stage alignment");
+constexpr int GROUP = 37;  // blocks that share a run of a batch's tiles
 constexpr int SMEM_LIMIT = 227 * 1024;  // per block
 static_assert(SMEM <= SMEM_LIMIT, "shared memory per block");
 }  // namespace tile
@@ -902,6 +903,28 @@ struct OneEventTiles {
     __device__ __forceinline__ float *phi_out_of(int) const { return phi_out; }
 };
 
+// A block's share of a batch's tiles: groups of `group` blocks (the last takes
+// the rest) each own a run of the list, and a group's blocks take its tiles in
+// turn. A block then meets few events, whose tensor maps it has to acquire, and
+// neighbouring tile rows are still worked on at the same time, so that their
+// halos are in L2. ms for 52 steps of 64 x 256^2 + 16 x 512^2 and of 10 x 64^2 +
+// 4 x 256^2: FP64 (444 blocks) in groups of 12, 37, 74, 148, 444: 124.4, 123.6,
+// 126.0, 125.7, 129.7 and 4.71, 4.73, 4.89, 4.73, 5.56; FP32 (148 blocks) in
+// groups of 12, 24, 37, 74, 148: 63.2, 63.2, 60.6, 64.1, 67.5 and 2.69, 2.85,
+// 2.83, 2.73, 2.94.
+struct TileShare {
+    int first, end, step;
+    __device__ __forceinline__ TileShare(int total, int group) {
+        const int blocks = gridDim.x, groups = blocks > group ? blocks / group : 1;
+        int g = blockIdx.x / group;
+        if (g >= groups) g = groups - 1;
+        const int b0 = g * group, b1 = g == groups - 1 ? blocks : b0 + group;
+        first = (int)((long long)total * b0 / blocks) + ((int)blockIdx.x - b0);
+        end = (int)((long long)total * b1 / blocks);
+        step = b1 - b0;
+    }
+};
+
 struct BatchTiles {
     const BatchEvent<float> *ev;  // shared memory
     const int *begin;             // shared memory, [n_events + 1]
@@ -997,7 +1020,11 @@ __device__ __forceinline__ void tile32_loop(const Tiles &T, unsigned char *smem,
     }
     allow_next_kernel();
     wait_previous_kernel();
-    const int first = blockIdx.x, end = T.total, step = gridDim.x;
+    int first = blockIdx.x, end = T.total, step = gridDim.x;
+    if constexpr (kLanes) {
+        const TileShare share(T.total, tile::GROUP);
+        first = share.first, end = share.end, step = share.step;
+    }
     if (issuer) {
         if (first < end) issue(first, 0);
         if (first + step < end) issue(first + step, 1);
@@ -1125,6 +1152,7 @@ constexpr uint32_t TX_BYTES = 2 * 9 * kU * 16 + 9 * kP * 8 + 2 * 8 * kS * 8 + 9 
 constexpr int SMEM = STAGE + 64 + 128;
 constexpr int THREADS = 2 * R * Cn;
 constexpr int BLOCKS = 3;  // per SM
+constexpr int GROUP = 37;  // blocks that share a run of the batch's tiles
 static_assert(BLOCKS * (SMEM + 1024) <= 228 * 1024, "shared memory of the SM");
 }  // namespace tile64
 
@@ -1343,16 +1371,17 @@ __global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
     compute_stage64(smem, ix0, iy0, cf, s, ux_out, uy_out, phi_out, N);
 }
 
-// The FP64 batch over the TMA tiles: BLOCKS persistent blocks an SM, each with
-// consecutive tiles of the concatenated tile lists, so that it meets few events:
-// a new event costs the acquire of its tensor maps in global memory. The step's
+// The FP64 batch over the TMA tiles: BLOCKS persistent blocks an SM, a new event
+// costs a block the acquire of its tensor maps (TileShare). The step's
 // descriptors and the tile prefix sums are copied to shared memory behind the
 // stage, since a thread reads its coefficients in the middle of the update.
 // ms for 52 steps of 3 x 512^2 + 8 x 128^2, 4 x 512^2 + 2 x 128^2 and
 // 4 x 256^2 + 10 x 64^2: one block per tile with its own acquires and
 // descriptor reads 21.5, 25.3, 7.3; persistent blocks on every gridDim.x-th
 // tile 15.6, 17.5, 6.1; consecutive tiles 14.9, 17.4, 5.4; descriptors in
-// shared memory as well 13.5, 15.7, 4.8.
+// shared memory as well 13.5, 15.7, 4.8; shares by groups 13.4, -, 4.7 (and
+// 64 x 256^2 + 16 x 512^2 133 -> 124, where consecutive tiles read the rows of
+// links between two tile rows from DRAM twice).
 __global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
     k_leapfrog_tile64_batch(const BatchEvent<double> *__restrict__ evs, int n_events,
                             const int *__restrict__ tile_begin, int total_tiles,
@@ -1380,8 +1409,8 @@ __global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
     wait_previous_kernel();
     uint32_t phase = 0;
     int e = 0, fenced = -1;
-    const int end = (int)((long long)total_tiles * (blockIdx.x + 1) / gridDim.x);
-    for (int t = (int)((long long)total_tiles * blockIdx.x / gridDim.x); t < end; t++) {
+    const TileShare share(total_tiles, tile64::GROUP);
+    for (int t = share.first; t < share.end; t += share.step) {
         while (s_begin[e + 1] <= t) e++;
         const BatchEvent<double> &E = s_ev[e];
         if (!E.active) continue;
