@@ -1153,7 +1153,14 @@ constexpr int SMEM = STAGE + 64 + 128;
 constexpr int THREADS = 2 * R * Cn;
 constexpr int BLOCKS = 3;  // per SM
 constexpr int GROUP = 37;  // blocks that share a run of the batch's tiles
-static_assert(BLOCKS * (SMEM + 1024) <= 228 * 1024, "shared memory of the SM");
+// events whose descriptors a batch block holds at a time: what three blocks an
+// SM leave room for
+constexpr int WINDOW = 87;
+// the batch kernel's block: the stage and its barrier, then the window's
+// descriptors and tile prefix sums
+constexpr int BATCH_SMEM =
+    SMEM + WINDOW * (int)sizeof(BatchEvent<double>) + (WINDOW + 1) * (int)sizeof(int);
+static_assert(BLOCKS * (BATCH_SMEM + 1024) <= 228 * 1024, "shared memory of the SM");
 }  // namespace tile64
 
 // Explicit shared-memory loads by 32-bit address, so that a link used twice
@@ -1372,9 +1379,15 @@ __global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
 }
 
 // The FP64 batch over the TMA tiles: BLOCKS persistent blocks an SM, a new event
-// costs a block the acquire of its tensor maps (TileShare). The step's
-// descriptors and the tile prefix sums are copied to shared memory behind the
-// stage, since a thread reads its coefficients in the middle of the update.
+// costs a block the acquire of its tensor maps (TileShare). Descriptors and
+// tile prefix sums are copied to shared memory behind the stage, since a thread
+// reads its coefficients in the middle of the update: WINDOW events at
+// a time, so that three blocks share an SM whatever the number of events. With
+// all events' descriptors in every block two blocks fitted from 88 events, one
+// from 325 and none from 1037; ms for 51 steps so and with the window: 80, 100
+// and 330 events of 64^2 5.27 -> 5.29, 9.36 -> 6.58 and 36.6 -> 20.0, 100 of
+// 256^2 126 -> 96. (One loop over all tiles that moved the window on inside
+// cost 1 to 2 % at 80 events of 64^2.)
 // ms for 52 steps of 3 x 512^2 + 8 x 128^2, 4 x 512^2 + 2 x 128^2 and
 // 4 x 256^2 + 10 x 64^2: one block per tile with its own acquires and
 // descriptor reads 21.5, 25.3, 7.3; persistent blocks on every gridDim.x-th
@@ -1392,49 +1405,71 @@ __global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + tile64::STAGE);
     BatchEvent<double> *s_ev =
         reinterpret_cast<BatchEvent<double> *>(smem + tile64::STAGE + 64);
-    int *s_begin = reinterpret_cast<int *>(s_ev + n_events);
-    {
-        const int words = n_events * (int)(sizeof(BatchEvent<double>) / sizeof(int));
-        const int *src = reinterpret_cast<const int *>(evs);
-        int *dst = reinterpret_cast<int *>(s_ev);
-        for (int w = threadIdx.x; w < words; w += tile64::THREADS) dst[w] = src[w];
-    }
-    for (int e = threadIdx.x; e <= n_events; e += tile64::THREADS) s_begin[e] = tile_begin[e];
+    int *s_begin = reinterpret_cast<int *>(s_ev + tile64::WINDOW);
+    const TileShare share(total_tiles, tile64::GROUP);
+    int base = 0;  // first event of the window
     if (threadIdx.x == 0) {
         mbar_init(full, 1);
         fence_barrier_init();
     }
-    __syncthreads();
-    allow_next_kernel();
-    wait_previous_kernel();
+    if (n_events > tile64::WINDOW) {
+        // the first window begins with the event of the block's first tile,
+        // found by counting the events that begin at or before it
+        int begun = 0;
+        for (int e = threadIdx.x; e < n_events; e += tile64::THREADS)
+            begun += tile_begin[e] <= share.first;
+        begun = __reduce_add_sync(0xffffffffu, begun);
+        if ((threadIdx.x & 31) == 0) s_begin[threadIdx.x >> 5] = begun;
+        __syncthreads();
+        for (int w = 0; w < tile64::THREADS / 32; w++) base += s_begin[w];
+        base--;
+        __syncthreads();  // the counts are read
+    }
     uint32_t phase = 0;
-    int e = 0, fenced = -1;
-    const TileShare share(total_tiles, tile64::GROUP);
-    for (int t = share.first; t < share.end; t += share.step) {
-        while (s_begin[e + 1] <= t) e++;
-        const BatchEvent<double> &E = s_ev[e];
-        if (!E.active) continue;
-        const int N = E.N, tiles_y = N / tile64::Cn, local = t - s_begin[e];
-        const int iy0 = (local % tiles_y) * tile64::Cn, ix0 = (local / tiles_y) * tile64::R;
-        const int tid = threadIdx.x;
-        if (tid < 32) {
-            if (tid == 0) mbar_arrive_expect_tx(full, tile64::TX_BYTES);
-            __syncwarp();
-            if (tid < 6) {
-                const CUtensorMap *mine = &maps[2 * e + E.map_sel].ux + tid;
-                if (fenced != e) fence_map_acquire(mine);
-                fenced = e;
-                load_box64(smem, mine, tid, ix0, iy0, full);
+    for (int t = share.first;; base += tile64::WINDOW) {
+        const int held = min(tile64::WINDOW, n_events - base);
+        {
+            const int words = held * (int)(sizeof(BatchEvent<double>) / sizeof(int));
+            const int *src = reinterpret_cast<const int *>(evs + base);
+            int *dst = reinterpret_cast<int *>(s_ev);
+            for (int w = threadIdx.x; w < words; w += tile64::THREADS) dst[w] = src[w];
+        }
+        for (int e = threadIdx.x; e <= held; e += tile64::THREADS) s_begin[e] = tile_begin[base + e];
+        __syncthreads();
+        if (t == share.first) {
+            allow_next_kernel();
+            wait_previous_kernel();
+        }
+        int e = 0, fenced = -1;
+        const int end = min(share.end, s_begin[held]);
+        for (; t < end; t += share.step) {
+            while (s_begin[e + 1] <= t) e++;
+            const BatchEvent<double> &E = s_ev[e];
+            if (!E.active) continue;
+            const int N = E.N, tiles_y = N / tile64::Cn, local = t - s_begin[e];
+            const int iy0 = (local % tiles_y) * tile64::Cn, ix0 = (local / tiles_y) * tile64::R;
+            const int tid = threadIdx.x;
+            if (tid < 32) {
+                if (tid == 0) mbar_arrive_expect_tx(full, tile64::TX_BYTES);
+                __syncwarp();
+                if (tid < 6) {
+                    const CUtensorMap *mine = &maps[2 * (base + e) + E.map_sel].ux + tid;
+                    if (fenced != e) fence_map_acquire(mine);
+                    fenced = e;
+                    load_box64(smem, mine, tid, ix0, iy0, full);
+                }
+            }
+            const bool arrived = mbar_wait_bounded(full, phase, tile::MAX_POLLS);
+            phase ^= 1;
+            if (arrived)
+                compute_stage64(smem, ix0, iy0, E.cf, E.s, E.ux_out, E.uy_out, E.phi_out, N);
+            if (__syncthreads_or(!arrived)) {  // else the stage is free
+                if (threadIdx.x == 0 && status) *status = 1.0;
+                return;
             }
         }
-        const bool arrived = mbar_wait_bounded(full, phase, tile::MAX_POLLS);
-        phase ^= 1;
-        if (arrived)
-            compute_stage64(smem, ix0, iy0, E.cf, E.s, E.ux_out, E.uy_out, E.phi_out, N);
-        if (__syncthreads_or(!arrived)) {  // else the stage is free
-            if (threadIdx.x == 0 && status) *status = 1.0;
-            return;
-        }
+        if (t >= share.end) return;
+        __syncthreads();  // no thread reads this window any more
     }
 }
 
@@ -1512,11 +1547,6 @@ size_t batch_smem(int n_events) {
     return sizeof(BatchEvent<T>) * n_events + sizeof(int) * (n_events + 1);
 }
 
-// shared memory of the FP64 tile batch kernel, in the same way: one stage
-size_t tile64_batch_smem(int n_events) {
-    return (size_t)tile64::SMEM + batch_smem<double>(n_events);
-}
-
 // shared memory of the FP32 TMA batch kernel: two stages, the barriers, the
 // descriptors and tile prefix sums, alignment slack
 size_t tile_batch_smem(int n_events) {
@@ -1549,10 +1579,8 @@ int batch_max_blocks_per_sm(int variant, int n_events) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile_batch, 256, smem);
             return nb > 1 ? 1 : nb;  // persistent: one block per SM
         } else {
-            const size_t smem = tile64_batch_smem(n_events);
-            if (smem > tile::SMEM_LIMIT) return 0;  // too many events for the descriptors
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile64_batch,
-                                                          tile64::THREADS, smem);
+                                                          tile64::THREADS, tile64::BATCH_SMEM);
             return nb > 0 ? 1 : 0;  // launched with BLOCKS blocks an SM
         }
     }
@@ -1575,7 +1603,7 @@ void launch_leapfrog_batch(const BatchEvent<T> *d_evs, int n_events, const int *
         } else {
             const int blocks = tile64::BLOCKS * grid;
             launch_after(k_leapfrog_tile64_batch, blocks < total_tiles ? blocks : total_tiles,
-                         tile64::THREADS, tile64_batch_smem(n_events), st, d_evs, n_events, d_tile_begin,
+                         tile64::THREADS, tile64::BATCH_SMEM, st, d_evs, n_events, d_tile_begin,
                          total_tiles, d_maps, status);
         }
         return;
@@ -1738,7 +1766,7 @@ cudaError_t prepare_leapfrog() {
         {(const void *)k_leapfrog_tile, tile::SMEM},
         {(const void *)k_leapfrog_tile64, tile64::SMEM},
         {(const void *)k_leapfrog_tile_batch, tile::SMEM_LIMIT},
-        {(const void *)k_leapfrog_tile64_batch, tile::SMEM_LIMIT}};
+        {(const void *)k_leapfrog_tile64_batch, tile64::BATCH_SMEM}};
     for (auto &k : kernels) {
         const cudaError_t e =
             cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, k.second);
