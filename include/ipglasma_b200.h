@@ -493,9 +493,10 @@ typedef struct ipg_batch ipg_batch;
 typedef struct {
     int variant;            /* tile-shape variant */
     int tile_rows;          /* a tile is 32 sites along y x tile_rows along x */
-    int threads_per_block;  /* one thread per site */
+    int threads_per_block;  /* one thread per site; FP64 TMA tile kernel: two */
     int blocks_per_sm;      /* resident blocks of the persistent grid */
-    int grid;               /* blocks_per_sm x SM count */
+    int grid;               /* blocks_per_sm x SM count (the TMA tile kernels
+                               launch at most one block a tile) */
     double ms_per_step;     /* measured time of one full step of the batch */
     int candidates;         /* shapes timed (0 when taken from the cache) */
     int from_cache;         /* 1 if the shape came from the tuning cache */
@@ -522,7 +523,9 @@ ipg_status ipg_batch_run(ipg_batch *batch, ipg_result *results);
 /* Set the launch shape by hand: variants 0, 1, 2 (FP32) or 0, 1 (FP64) are
  * plain-load kernels on tiles of 2, 4 or 8 rows; variant 3 (FP32) or 2 (FP64)
  * is the TMA tile kernel of the single-event form run over every event's
- * tiles (1 block per SM); 1 <= blocks_per_sm <= what fits on an SM. */
+ * tiles. Plain kernels: 1 <= blocks_per_sm <= what fits on an SM. TMA tile
+ * kernel: 1 or the count of its tune report; it runs on its own count (1 block
+ * per SM in FP32, 3 in FP64) either way. */
 ipg_status ipg_batch_set_shape(ipg_batch *batch, int variant, int blocks_per_sm);
 ipg_status ipg_batch_stats(const ipg_batch *batch, double *ms_evolution,
                            double *ms_total, long long *launches);

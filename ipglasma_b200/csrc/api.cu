@@ -2408,6 +2408,14 @@ int tma_variant(const ipg_batch *b) {
     return b->fp32 ? batch_plain_variants<float>() : batch_plain_variants<double>();
 }
 
+// The launch shape from now on. The TMA tile kernels always take the blocks an
+// SM that their shared memory allows, whatever count was asked for or saved.
+void use_shape(ipg_batch *b, int variant, int blocks_per_sm) {
+    b->variant = variant;
+    b->blocks_per_sm = variant == tma_variant(b) ? max_blocks(b, variant) : blocks_per_sm;
+    b->grid = b->blocks_per_sm * b->sms;
+}
+
 // whether (variant, blocks per SM) can run this batch
 bool shape_fits(const ipg_batch *b, const std::pair<int, int> &shape) {
     const int v = shape.first;
@@ -2629,21 +2637,15 @@ ipg_status ipg_batch_create(ipg_ctx *const *events, int count, ipg_batch **out) 
     const auto it = tune_cache().find(tune_key(b));
     // (a shape saved by another build may not fit this one's kernels)
     if (it != tune_cache().end() && shape_fits(b, it->second)) {
-        b->variant = it->second.first;
-        b->blocks_per_sm = it->second.second;
+        use_shape(b, it->second.first, it->second.second);
         b->tuned = true;
     } else {
         // the TMA tile kernel when the maps and the descriptors fit, else the
         // plain-load kernel with 4-row tiles
-        b->variant = tma_variant(b);
-        b->blocks_per_sm = b->d_maps ? max_blocks(b, b->variant) : 0;
-        if (b->blocks_per_sm < 1) {
-            b->variant = 1;
-            b->blocks_per_sm = max_blocks(b, b->variant);
-        }
+        const int v = b->d_maps && max_blocks(b, tma_variant(b)) > 0 ? tma_variant(b) : 1;
+        use_shape(b, v, max_blocks(b, v));
     }
     if (b->blocks_per_sm < 1) return bfail(b, IPG_ERR_CUDA, "batched kernel cannot be resident");
-    b->grid = b->blocks_per_sm * b->sms;
     return IPG_OK;
 }
 
@@ -2695,7 +2697,8 @@ ipg_status ipg_batch_tune(ipg_batch *b, ipg_tune_report *rep) {
         if (!rep) return;
         rep->variant = b->variant;
         rep->tile_rows = tile_rows(b, b->variant);
-        rep->threads_per_block = 32 * rep->tile_rows;
+        rep->threads_per_block = b->fp32 ? batch_threads<float>(b->variant)
+                                         : batch_threads<double>(b->variant);
         rep->blocks_per_sm = b->blocks_per_sm;
         rep->grid = b->grid;
         rep->ms_per_step = ms;
@@ -2704,9 +2707,7 @@ ipg_status ipg_batch_tune(ipg_batch *b, ipg_tune_report *rep) {
     };
     auto hit = tune_cache().find(key);
     if (hit != tune_cache().end() && shape_fits(b, hit->second)) {
-        b->variant = hit->second.first;
-        b->blocks_per_sm = hit->second.second;
-        b->grid = b->blocks_per_sm * b->sms;
+        use_shape(b, hit->second.first, hit->second.second);
         b->tuned = true;
         fill_report(0., 0, 1);
         return IPG_OK;
@@ -2746,10 +2747,8 @@ ipg_status ipg_batch_tune(ipg_batch *b, ipg_tune_report *rep) {
     int best_v = b->variant, best_bps = b->blocks_per_sm, candidates = 0;
     for (int v = 0; v < n_variants(b); v++) {
         const int maxb = (v == tma_variant(b) && !b->d_maps) ? 0 : max_blocks(b, v);
-        for (int bps = 1; bps <= maxb; bps++) {
-            b->variant = v;
-            b->blocks_per_sm = bps;
-            b->grid = bps * b->sms;
+        for (int bps = v == tma_variant(b) ? std::max(1, maxb) : 1; bps <= maxb; bps++) {
+            use_shape(b, v, bps);
             IPG_TRY(upload_tiles(b, v));
             launch_batch(b, slot);  // warm-up
             IPG_BCUDA(b, cudaEventRecord(b->e0, b->stream));
@@ -2781,9 +2780,7 @@ ipg_status ipg_batch_tune(ipg_batch *b, ipg_tune_report *rep) {
     }
     IPG_BCUDA(b, cudaStreamSynchronize(b->stream));
     for (void *q : saved) cudaFree(q);
-    b->variant = best_v;
-    b->blocks_per_sm = best_bps;
-    b->grid = best_bps * b->sms;
+    use_shape(b, best_v, best_bps);
     b->tuned = true;
     tune_cache()[key] = {best_v, best_bps};
     if (const char *path = std::getenv("IPG_TUNE_CACHE")) {
@@ -2863,11 +2860,15 @@ ipg_status ipg_batch_set_shape(ipg_batch *b, int variant, int blocks_per_sm) {
     if (variant < 0 || variant >= n_variants(b) || (variant == tma_variant(b) && !b->d_maps))
         return bfail(b, IPG_ERR_BAD_CONFIG, "variant %d not available", variant);
     const int maxb = max_blocks(b, variant);
-    if (blocks_per_sm < 1 || blocks_per_sm > maxb)
+    if (variant == tma_variant(b)) {
+        // 1 stands for the kernel's own count; the count that a tune report
+        // gives for it is taken too
+        if (maxb < 1 || (blocks_per_sm != 1 && blocks_per_sm != maxb))
+            return bfail(b, IPG_ERR_BAD_CONFIG, "variant %d runs %d blocks an SM", variant, maxb);
+    } else if (blocks_per_sm < 1 || blocks_per_sm > maxb) {
         return bfail(b, IPG_ERR_BAD_CONFIG, "blocks_per_sm must be in [1, %d]", maxb);
-    b->variant = variant;
-    b->blocks_per_sm = blocks_per_sm;
-    b->grid = blocks_per_sm * b->sms;
+    }
+    use_shape(b, variant, blocks_per_sm);
     return IPG_OK;
 }
 

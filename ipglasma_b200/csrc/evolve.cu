@@ -1561,6 +1561,12 @@ int batch_tile_rows(int variant) {
 }
 
 template <typename T>
+int batch_threads(int variant) {
+    if (sizeof(T) == 8 && variant == batch_plain_variants<T>()) return tile64::THREADS;
+    return 32 * batch_tile_rows<T>(variant);
+}
+
+template <typename T>
 const void *batch_kernel(int variant) {
     switch (variant) {
         case 0: return (const void *)k_leapfrog_batch<2, T>;
@@ -1581,10 +1587,10 @@ int batch_max_blocks_per_sm(int variant, int n_events) {
         } else {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_leapfrog_tile64_batch,
                                                           tile64::THREADS, tile64::BATCH_SMEM);
-            return nb > 0 ? 1 : 0;  // launched with BLOCKS blocks an SM
+            return nb < tile64::BLOCKS ? nb : tile64::BLOCKS;
         }
     }
-    const int threads = 32 * batch_tile_rows<T>(variant);
+    const int threads = batch_threads<T>(variant);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_kernel<T>(variant), threads,
                                                   batch_smem<T>(n_events));
     return nb;
@@ -1601,8 +1607,7 @@ void launch_leapfrog_batch(const BatchEvent<T> *d_evs, int n_events, const int *
             launch_after(k_leapfrog_tile_batch, grid < total_tiles ? grid : total_tiles, 256, smem,
                          st, d_evs, n_events, d_tile_begin, total_tiles, d_maps, status, 4u);
         } else {
-            const int blocks = tile64::BLOCKS * grid;
-            launch_after(k_leapfrog_tile64_batch, blocks < total_tiles ? blocks : total_tiles,
+            launch_after(k_leapfrog_tile64_batch, grid < total_tiles ? grid : total_tiles,
                          tile64::THREADS, tile64::BATCH_SMEM, st, d_evs, n_events, d_tile_begin,
                          total_tiles, d_maps, status);
         }
@@ -1627,6 +1632,8 @@ void launch_leapfrog_batch(const BatchEvent<T> *d_evs, int n_events, const int *
 
 template int batch_tile_rows<float>(int);
 template int batch_tile_rows<double>(int);
+template int batch_threads<float>(int);
+template int batch_threads<double>(int);
 template int batch_max_blocks_per_sm<float>(int, int);
 template int batch_max_blocks_per_sm<double>(int, int);
 template void launch_leapfrog_batch<float>(const BatchEvent<float> *, int, const int *, int,

@@ -94,7 +94,8 @@ bool encode_step_maps<double>(int N, const State<double> &s, LoadMaps *out);
 // advances tiles of 32 x batch_tile_rows(v) sites with plain loads, one
 // thread per site; the last variant (v = batch_plain_variants) runs the TMA
 // tile kernel of the single-event form over the concatenated tile lists,
-// with per-event tensor maps (d_maps[2 e + map_sel]).
+// with per-event tensor maps (d_maps[2 e + map_sel]), on as many blocks an SM
+// as batch_max_blocks_per_sm gives for it (FP32 one, FP64 three).
 template <typename T>
 constexpr int batch_plain_variants() {
     return sizeof(T) == 4 ? 3 : 2;
@@ -105,6 +106,8 @@ constexpr int batch_variants() {
 }
 template <typename T>
 int batch_tile_rows(int variant);
+template <typename T>
+int batch_threads(int variant);  // per block
 template <typename T>
 int batch_max_blocks_per_sm(int variant, int n_events);
 // tile_begin[n_events + 1]: prefix sums of (N/32) (N/rows) per event;
