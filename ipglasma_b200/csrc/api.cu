@@ -63,7 +63,9 @@ struct ipg_ctx {
     // FP32 (the transforms of the FP32 form run in FP32)
     float2 *twiddle32 = nullptr;
     float *green32 = nullptr;
-    double *amp = nullptr, *ampB = nullptr;  // charge amplitudes of A and B
+    // charge amplitudes of A, and of B where both are worked on at a time (the
+    // nuclei's lines side by side, the input adjoint)
+    double *amp = nullptr, *ampB = nullptr;
     double2 *work = nullptr, *work2 = nullptr;
     double *nuc_xyz = nullptr, *nuc_gx = nullptr, *nuc_gy = nullptr;  // ipg_set_nuclei
     struct {  // ipg_set_nuclei_ipsat (allocated by its first call)
@@ -259,6 +261,12 @@ ipg_status alloc_state32(ipg_ctx *c, State<float> &s) {
 }
 
 bool is_fp32(const ipg_ctx *c) { return c->cfg.precision == IPG_FP32; }
+
+// sheets of a batch of the Wilson-line stage: the FP32 form transforms in FP32,
+// twice the sheets fit a work buffer
+int sheets_a_batch(const ipg_ctx *c) { return is_fp32(c) ? 2 * c->work_sheets : c->work_sheets; }
+// whether the two nuclei's lines run side by side (init_enqueue)
+bool nuclei_side_by_side(const ipg_ctx *c) { return c->cfg.Ny <= sheets_a_batch(c); }
 
 // one leapfrog launch on the active precision, then swap the U/phi buffers
 template <typename T>
@@ -837,7 +845,6 @@ ipg_status ipg_create(const ipg_config *cfg, ipg_ctx **out) {
     IPG_TRY(dalloc(c, &c->twiddle, (size_t)N));
     IPG_TRY(dalloc(c, &c->green, n));
     IPG_TRY(dalloc(c, &c->amp, n));
-    IPG_TRY(dalloc(c, &c->ampB, n));
     // work buffer of a sheet batch: up to 128 MB (8 sheets at 512^2, 32 at
     // 256^2). Larger batches give each transform launch more parallelism:
     // the 512^2 Wilson-line stage takes 3.59 ms at 128 MB, 3.68 ms at 64 MB,
@@ -845,6 +852,7 @@ ipg_status ipg_create(const ipg_config *cfg, ipg_ctx **out) {
     const size_t per_sheet = 4 * n * sizeof(double2);
     c->work_sheets = (int)std::max<size_t>(1, (128ull << 20) / per_sheet);
     c->work_sheets = std::min(c->work_sheets, cfg->Ny);
+    if (nuclei_side_by_side(c)) IPG_TRY(dalloc(c, &c->ampB, n));
     IPG_TRY(dalloc(c, &c->work, (size_t)c->work_sheets * 4 * n));
     IPG_TRY(dalloc(c, &c->work2, (size_t)c->work_sheets * 4 * n));
     IPG_TRY(dalloc(c, &c->VA, 9 * n));
@@ -1306,8 +1314,7 @@ static ipg_status init_enqueue(ipg_ctx *c, bool from_wilson) {
     // 128^2 206 -> 172, 256^2 614 -> 588, 512^2 (16 sheets) 758 -> 728). Several
     // batches a nucleus already run the products of one beside the transforms
     // of the next.
-    const int sheets_a_batch = is_fp32(c) ? 2 * c->work_sheets : c->work_sheets;
-    const bool side_by_side = !from_wilson && c->cfg.Ny <= sheets_a_batch;
+    const bool side_by_side = !from_wilson && nuclei_side_by_side(c);
     if (side_by_side) {
         IPG_CUDA(c, cudaEventRecord(c->ev_nuc_fork, c->stream));
         IPG_CUDA(c, cudaStreamWaitEvent(c->stream_v, c->ev_nuc_fork, 0));
@@ -1329,14 +1336,13 @@ static ipg_status init_enqueue(ipg_ctx *c, bool from_wilson) {
         w.nucleus = (uint32_t)nuc;
         w.twiddle = c->twiddle;
         w.green = c->green;
-        w.amp = nuc ? c->ampB : c->amp;
+        w.amp = nuc && side_by_side ? c->ampB : c->amp;
         w.work = c->work;
         w.V = V;
-        // the FP32 form transforms in FP32: twice the sheets fit a work buffer
         w.fp32 = is_fp32(c) ? 1 : 0;
         w.twiddle32 = c->twiddle32;
         w.green32 = c->green32;
-        const int sheets = sheets_a_batch;
+        const int sheets = sheets_a_batch(c);
         launch_wilson_amp(w, st);
         IPG_LAUNCHED(c, 1);
         if (side_by_side) {
@@ -1893,6 +1899,7 @@ ipg_status backward_inputs(ipg_ctx *c, double *grad_g2mu, double *grad_rho) {
             IPG_TRY(dalloc(c, p, 9 * n));
         IPG_TRY(dalloc(c, &A.g2mu_bar, 2 * n));
     }
+    if (!c->ampB) IPG_TRY(dalloc(c, &c->ampB, n));
     if (grad_rho && !A.rho_all) IPG_TRY(dalloc(c, &A.rho_all, 16 * (size_t)Ny * n));
     for (C<double> *p : {A.b1x, A.b2x, A.b1y, A.b2y, A.vbA, A.vbB})
         IPG_CUDA(c, cudaMemsetAsync(p, 0, 9 * n * sizeof(C<double>), c->stream));
