@@ -142,8 +142,6 @@ __device__ __forceinline__ void restart_alpha(double alpha[8], uint64_t key,
 constexpr int kNewtonThreads = 128;
 // doubles of shared memory per thread: J (64), F, dalpha, alpha, best alpha
 constexpr int kNewtonSmem = 64 + 4 * 8;
-constexpr int kNewtonFirst = 8 * 18;  // doubles per block: the first Jacobian's exponentials
-constexpr double kFirstStep = 0.001;  // the difference step at alpha = 0 (Init.cpp:3380-3470)
 
 // the exponent held in shared memory, into registers, entry b replaced by v
 __device__ __forceinline__ void load_alpha(const double *al, int js, double out[8], int b = -1,
@@ -196,33 +194,7 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
     double *Fa = J + 64 * js, *dalpha = J + 72 * js, *al = J + 80 * js, *best_al = J + 88 * js;
     const size_t n = (size_t)A.N * A.N;
     const size_t lid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool mine = lid < 2 * n && !(A.redo_only && A.status[lid] != -1);
-    // The iteration starts at alpha = 0, where the differenced exponentials of
-    // the first Jacobian are exp(i 0.001 t^b) for every link: eight threads
-    // evaluate them for the block (a link takes 1.5 iterations at 512^2, 3.7 at
-    // 64^2)
-    double *first = newton_j + kNewtonSmem * js;
-    if (!__syncthreads_or(mine)) return;
-    if (threadIdx.x < 8) {
-        double q[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) q[k] = k == (int)threadIdx.x ? kFirstStep : 0.;
-        const M3<double> e = exp_from_coeff(q);
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            first[18 * threadIdx.x + 2 * k] = e.m[k].r;
-            first[18 * threadIdx.x + 2 * k + 1] = e.m[k].i;
-        }
-    }
-    __syncthreads();
-    if (!mine) return;
-    // Where the last of them is the identity (the closed form gives that for
-    // exactly coinciding eigenvalues), its column of the first Jacobian is zero
-    // and the iteration takes the analytic one whatever the others are
-    bool first_good = false;
-#pragma unroll
-    for (int k = 0; k < 18; k++)
-        first_good = first_good || first[18 * 7 + k] != ((k == 0 || k == 8 || k == 16) ? 1. : 0.);
+    if (lid >= 2 * n || (A.redo_only && A.status[lid] != -1)) return;
     // link order of the reference loop: per site, x then y (Init.cpp:2498-2516)
     const size_t pos = lid >> 1;
     const int dir = (int)(lid & 1);
@@ -263,22 +235,20 @@ __global__ void __launch_bounds__(kNewtonThreads) k_newton(NewtonArgs A) {
                 Fzero += fabs(f);
             }
         }
-        bool good = total > 1 || first_good;
-        for (int b = 0; b < 8 && (total > 1 || first_good); b++) {
+        // At alpha = 0, where the iteration starts, the differenced exponentials
+        // are those of 0.001 t^b for every link. The closed form gives exactly
+        // the identity for the last of them (t^8 has two equal eigenvalues, and
+        // c0 / c0max comes out as -1 - 4e-16, which has no arc cosine), so its
+        // column is zero and the first Jacobian is the analytic one, without any
+        // difference.
+        bool good = total > 1;
+        for (int b = 0; b < 8 && total > 1; b++) {
             const double ab = al[b * js];
-            const double d = fmax(kFirstStep, fmin(10., 0.01 * fabs(ab)));
+            const double d = fmax(0.001, fmin(10., 0.01 * fabs(ab)));
             const double ap = ab + d;
-            M3<double> E1;
-            if (total == 1) {
-#pragma unroll
-                for (int k = 0; k < 9; k++)
-                    E1.m[k] = {first[18 * b + 2 * k], first[18 * b + 2 * k + 1]};
-            } else {
-                load_alpha(al, js, a8, b, ap);
-                E1 = exp_from_coeff(a8);
-            }
+            load_alpha(al, js, a8, b, ap);
             double tl[8];
-            L.difference(E1, tl);
+            L.difference(exp_from_coeff(a8), tl);
             double mcheck = 0.;
 #pragma unroll
             for (int a = 0; a < 8; a++) {
@@ -502,8 +472,7 @@ __global__ void __launch_bounds__(kFastThreads) k_newton_fast(NewtonArgs A) {
 void launch_newton(const NewtonArgs &a, cudaStream_t st) {
     const size_t links = 2 * (size_t)a.N * a.N;
     const unsigned blocks = (unsigned)((links + kNewtonThreads - 1) / kNewtonThreads);
-    // 97 KB: two blocks an SM
-    const size_t smem = sizeof(double) * (kNewtonSmem * kNewtonThreads + kNewtonFirst);
+    const size_t smem = sizeof(double) * kNewtonSmem * kNewtonThreads;  // 96 KB: two blocks an SM
     cudaFuncSetAttribute(k_newton, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     NewtonArgs b = a;
     if (a.mode == 1) {
