@@ -486,6 +486,7 @@ ipg_status ipg_adjoint_stats(const ipg_ctx *ctx, double *ms_forward, double *ms_
  * sites of all events, and the whole step sequence is a CUDA graph captured
  * on the first run and replayed afterwards. This is the multi-event form of
  * "ipg_evolve(ctx, ev_first, ev_count, nsteps)": each context is one event.
+ * An FP32 batch holds at most 372 events, an FP64 batch any number.
  * The batch does not own its contexts; destroy it before them. */
 typedef struct ipg_batch ipg_batch;
 

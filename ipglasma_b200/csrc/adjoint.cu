@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(128, 3) k_inv_adj_su(int N, State<T> nxt, Stat
 // role 2: Ux(-x) += Uy(-x) Qb2 + 2 phi(-x) Ux(-x) brb; Uy(-x) += Ux(-x) Qb2^dag;
 //         phi(-x) += Ux(-x) brb Ux(-x)^dag; and the same along y with Qb
 //
-// FP32: four blocks an SM (128 registers, 116 B of spill) against three
+// FP32: four blocks an SM (128 registers, 88 B of spill) against three
 // unbounded (168): 70 against 74 us a checkpointed backward step at 256^2, 154
 // against 160 us at 512^2 with every state kept. FP64 stays unbounded (255):
 // at 168 registers it spills 1 KB, 293 against 278 us at 512^2.

@@ -622,7 +622,7 @@ struct PairLoadGlobal {
 // returns the new links (nu) and phi (phin) when cf.do_pu is set, for the
 // caller to store once no other thread reads the old ones. The site's own
 // link pair is loaded again at each use instead of being held (the tile
-// kernel then fits in 252 registers without spilling).
+// kernel then fits in 254 registers without spilling).
 template <class Ld>
 __device__ __forceinline__ void leapfrog_pair_core(const Ld &ld, const StepCoef<float> &cf,
                                                    M3<P2> &nu, H3<float> &phin) {
@@ -734,7 +734,7 @@ constexpr uint32_t TX_BYTES = 2 * 9 * kU * 8 + 9 * kP * 4 + 2 * 8 * kS * 4 + 9 *
 constexpr int SMEM = 2 * STAGE + 64 + 128;  // two stages, four barriers, alignment slack
 constexpr uint32_t MAX_POLLS = 1u << 22;
 static_assert(STAGE % 128 == 0, "stage alignment");
-constexpr int GROUP = 37;  // blocks that share a run of a batch's tiles
+constexpr int GROUP = 37;  // blocks that share a run of a batch's tiles (a quarter of the 148)
 constexpr int SMEM_LIMIT = 227 * 1024;  // per block
 static_assert(SMEM <= SMEM_LIMIT, "shared memory per block");
 }  // namespace tile
@@ -911,7 +911,9 @@ struct OneEventTiles {
 // 4 x 256^2: FP64 (444 blocks) in groups of 12, 37, 74, 148, 444: 124.4, 123.6,
 // 126.0, 125.7, 129.7 and 4.71, 4.73, 4.89, 4.73, 5.56; FP32 (148 blocks) in
 // groups of 12, 24, 37, 74, 148: 63.2, 63.2, 60.6, 64.1, 67.5 and 2.69, 2.85,
-// 2.83, 2.73, 2.94.
+// 2.83, 2.73, 2.94. 37 is taken for the large batches; the small FP32 batch
+// would be 5% faster in groups of 12. Not all halos are in L2: on the large batch
+// DRAM reads are 13% (FP32) and 19% (FP64) above the state.
 struct TileShare {
     int first, end, step;
     __device__ __forceinline__ TileShare(int total, int group) {
@@ -1123,14 +1125,15 @@ __global__ void __launch_bounds__(256, 1)
 // ---------------------------------------------------------------------------
 // FP64 step with the fields staged in shared memory by TMA: one block per
 // tile of 2 rows (x) x 32 columns (y), two threads per site (the x and the y
-// direction: lanes l and l + 16 of a warp share site l). A thread then fits
-// in 128 registers without spilling, and three 128-thread blocks (12 warps)
-// share an SM, some loading while others compute. The stage holds
+// direction: lanes l and l + 16 of a warp share site l). A thread then needs
+// 156 registers without spilling (168 in the batch kernel, the limit for three
+// blocks; one thread a site 190), and three 128-thread blocks (12 warps) share
+// an SM, some loading while others compute. The stage holds
 //   Ux, Uy   [9][4][34] complex  rows ix0-1 .. ix0+2, columns iy0-1 .. iy0+32
 //   phi      [9][4][36] real     rows ix0-1 .. ix0+2, columns iy0-2 .. iy0+33
 //   E1, E2   [8][2][32], pi [9][2][32]   the tile's own sites
 // Results go to global memory from registers (E and pi in place).
-// Bound by the FP64 pipe (about 60% busy at 512^2) and the wait for the
+// Bound by the FP64 pipe (60% of its cycles at 512^2) and the wait for the
 // stage. us a step at 64^2, 128^2, 256^2, 512^2, 1024^2: one thread a site on
 // 4 x 32 tiles 11.5, 12.3, 24.6, 77.0, 258.8; this kernel 6.2, 9.1, 18.8,
 // 65.3, 232.2 (before dependent launches). Tiles of 4 rows (two blocks an SM): 8.2, 9.0, 20.6, 67.2,
@@ -1152,7 +1155,7 @@ constexpr uint32_t TX_BYTES = 2 * 9 * kU * 16 + 9 * kP * 8 + 2 * 8 * kS * 8 + 9 
 constexpr int SMEM = STAGE + 64 + 128;
 constexpr int THREADS = 2 * R * Cn;
 constexpr int BLOCKS = 3;  // per SM
-constexpr int GROUP = 37;  // blocks that share a run of the batch's tiles
+constexpr int GROUP = 37;  // blocks that share a run of the batch's tiles (1/12 of 3 x 148)
 // events whose descriptors a batch block holds at a time: what three blocks an
 // SM leave room for
 constexpr int WINDOW = 87;
@@ -1339,7 +1342,7 @@ __device__ __forceinline__ void compute_stage64(const unsigned char *smem, int i
 }
 
 // One block per tile of the event's N/2 x N/32 grid.
-// (THREADS, 3): what shared memory allows, 168 registers a thread
+// (THREADS, 3): what shared memory allows; at most 168 registers a thread
 __global__ void __launch_bounds__(tile64::THREADS, tile64::BLOCKS)
     k_leapfrog_tile64(const __grid_constant__ LoadMaps maps, int N, StepCoef<double> cf,
                       double *status, State<double> s, C<double> *ux_out, C<double> *uy_out,

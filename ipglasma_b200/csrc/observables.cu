@@ -390,7 +390,7 @@ template <typename S>
 static int launch_tmunu_t(const TmunuArgs &a, cudaStream_t st) {
     const size_t n = (size_t)a.N * a.N;
     const unsigned b = (unsigned)((n + 127) / 128);
-    // side by side while one part does not give every SM a block: us for all
+    // side by side while one part does not give each of the 148 SMs a block: us for all
     // observables one after the other and side by side, 64^2 178 and 149, 128^2
     // 197 and 197; above that the mixed parts spill more and share the L1 worse:
     // 256^2 295 and 309, 512^2 FP32 854 and 872
